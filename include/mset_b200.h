@@ -159,10 +159,12 @@ int mset_adjoint_position(mset_session *s, int mode, int adjoint, const float *r
 int mset_read_state(mset_session *s, float *rvol_out, float *probe_out);
 /* The sequential pass (mset_run) and the per-position steps walk one position
  * at a time, so one position's field is all the parallel work there is.
- * Where a cluster geometry is compiled for the window (n = 128: 8 CTAs of 16
- * rows), that field is split over a thread-block cluster (distributed shared
- * memory) and each position runs on several SMs; results are those of the
- * one-CTA kernel up to the order of the cluster's partial sums.
+ * That field is spread over a thread-block cluster (n = 48, 64, 128: 8 CTAs;
+ * 96, 160, 256: 16; 24, 32: one CTA), whose CTAs exchange rows and columns
+ * through distributed shared memory; results are those of the one-CTA kernel
+ * up to the order of the FP64 partial sums.  The cluster kernels keep the
+ * transmission slabs as scratch ([ns][n][n] complex64); without memory for it
+ * the one-CTA kernel runs.
  * mset_set_sequential_split(s, 0) keeps one CTA per field; on by default.
  * mset_sequential_split returns the CTAs per field the sequential modes use. */
 int mset_set_sequential_split(mset_session *s, int on);

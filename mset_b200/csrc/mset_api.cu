@@ -106,11 +106,11 @@ struct mset_session {
     float sigma = 0, dz = 0, step[3] = {0, 0, 0};
     int nsx = 0, nsy = 0;
     Plan plan{};
-    // sequential modes (kSeq, kStep): one field split over a thread-block
-    // cluster, where such a geometry is compiled for n (seq_split: in use)
-    Plan seq_plan{};
-    bool has_seq = false;
+    // sequential modes (kSeq, kStep): the window's kernels on a cluster per
+    // field (seq_split: in use; kernels of one CTA per field always are)
+    const SeqOps *seq = nullptr;
     bool seq_split = true;
+    DevBuf<double> seq_part;  // their partial sums
     bool ready = false;
     bool batch = false;
     // tilts (1 for the MEX-style session)
@@ -218,17 +218,16 @@ int ensure_geometry(mset_session *s, int n, int nz, int b, float sigma, float dz
         return fail(MSET_E_UNSUPPORTED,
                     "window size %d has no compiled kernel (supported: 24, 32, 48, 64, 96, 128, 160, 256)", n);
     if (b > nz) b = nz;  // STEP00_INIT.m:126-128
-    Plan sq{};
-    bool has_seq = plan_seq_for(n, &sq);
-    if (sequential && has_seq && (sq.r1 != pl.r1 || sq.ry1 != pl.ry1)) {
+    const SeqOps *sq = sequential ? seq_ops_for(n) : nullptr;
+    if (sq && !sq->fits()) sq = nullptr;
+    if (sq && (sq->r1 != pl.r1 || sq->r1 != pl.ry1)) {
         Plan alt;
-        if (plan_for_layout(n, sq.r1, sq.ry1, &alt)) pl = alt;
+        if (plan_for_layout(n, sq->r1, sq->r1, &alt)) pl = alt;
+        else sq = nullptr;
     }
-    has_seq = has_seq && sq.r1 == pl.r1 && sq.ry1 == pl.ry1;
     if (pl.cl > 1) pl.max_clusters = pl.ops->max_clusters();
     s->plan = pl;
-    s->seq_plan = sq;
-    s->has_seq = has_seq;
+    s->seq = sq;
     s->n = n;
     s->nz = nz;
     s->b = b;
@@ -345,7 +344,9 @@ int upload_tilt_measured(mset_session *s, TiltBufs &t, const float *meas, const 
     return 0;
 }
 
-int refresh_tilt_table(mset_session *s) {
+// seq_t: hand the sequential tilt's transmission slabs to the kernel (the
+// others read the volume, which those kernels change)
+int refresh_tilt_table(mset_session *s, bool seq_t = false) {
     const int J = (int)s->tilts.size();
     s->h_tilts.assign(J, TiltDev{});
     for (int j = 0; j < J; ++j) {
@@ -362,7 +363,7 @@ int refresh_tilt_table(mset_session *s) {
         d.posdir = t.posdir.p;
         d.err = s->err.p + j;
         d.inten = s->inten.p ? s->inten.p + (size_t)s->pos_off[j] * s->n * s->n : nullptr;
-        d.T = s->batch ? t.T.p : nullptr;
+        d.T = s->batch || seq_t ? t.T.p : nullptr;
         d.npos = t.npos;
     }
     CK(s->d_tilts.ensure(J));
@@ -413,13 +414,55 @@ LaunchArgs base_args(mset_session *s) {
     return a;
 }
 
+// whether the sequential modes run on the cluster kernels
+bool seq_on_cluster(const mset_session *s) { return s->seq && (s->seq_split || s->seq->cl == 1); }
+
+// Before a sequential launch over npos positions of method: true where it runs
+// on the cluster kernels, whose scratch (transmission slabs, partial sums) is
+// then there.  Without the memory for it the one-CTA kernel runs, which reads
+// the volume.  Sets the tilt table.
+int seq_prepare(mset_session *s, int method, int npos, bool *cluster) {
+    const size_t n2 = (size_t)s->n * s->n;
+    *cluster = seq_on_cluster(s);
+    if (*cluster) {
+        TiltBufs &t = s->tilts[0];
+        const size_t parts = (size_t)(2 * std::max(1, npos) + 1) * s->seq->warps;
+        const size_t slabs = method == kSSET ? 1 : s->ns;
+        cudaError_t e = t.T.n < n2 * slabs ? t.T.ensure(n2 * s->ns) : cudaSuccess;
+        if (e == cudaSuccess && s->seq_part.n < parts) e = s->seq_part.ensure(parts);
+        if (e == cudaErrorMemoryAllocation && s->plan.ops->seq) {
+            cudaGetLastError();
+            *cluster = false;
+        } else if (e != cudaSuccess) {
+            return cuda_fail(e, "allocating the sequential pass's scratch");
+        }
+    }
+    return refresh_tilt_table(s, *cluster);
+}
+
+// the transmission slabs of the sequential tilt from its volume
+int seq_transmission(mset_session *s, int method) {
+    const bool sset = method == kSSET;
+    CKL(launch_transmission(s->d_tilts.p, 1, s->n, s->nz, sset ? s->nz : s->b, sset ? 1 : s->ns, s->sigma * s->dz,
+                            s->st),
+        "transmission");
+    return 0;
+}
+
+int launch_sequential(mset_session *s, bool cluster, int method, int adjoint, int mode, LaunchArgs &a,
+                      const char *what) {
+    if (cluster) {
+        a.seq_part = s->seq_part.p;
+        CKL(s->seq->positions(method, adjoint, mode, a, s->st), what);
+    } else {
+        CKL(launch_positions(s->plan, method, adjoint, mode, a, std::max(1, s->plan.cl), s->st), what);
+    }
+    return 0;
+}
+
 // The position kernel waits, with a bound, for the bulk copies that stage
 // its operands in shared memory; a wait that gave up sets the session's
 // fault word.  Read (and clear) it where a call hands results back.
-// the plan of the sequential modes: the cluster geometry when compiled and
-// enabled, else the session's own
-const Plan &seq_plan(const mset_session *s) { return (s->has_seq && s->seq_split) ? s->seq_plan : s->plan; }
-
 int take_fault(mset_session *s) {
     if (!s->fault.p) return 0;
     unsigned f = 0;
@@ -593,12 +636,14 @@ int mset_run_ex(mset_session *s, int mode, int adjoint, float *rvol_out, float *
     s->step_k = -1;
     rc = ensure_save(s, 1);
     if (rc) return rc;
-    rc = refresh_tilt_table(s);
+    TiltBufs &t = s->tilts[0];
+    bool cluster = false;
+    rc = seq_prepare(s, mode, t.npos, &cluster);
+    if (!rc && cluster) rc = seq_transmission(s, mode);
     if (rc) return rc;
     LaunchArgs a = base_args(s);
-    const Plan &sp = seq_plan(s);
-    CKL(launch_positions(sp, mode, adjoint, kSeq, a, std::max(1, sp.cl), s->st), "sequential position kernel launch");
-    TiltBufs &t = s->tilts[0];
+    rc = launch_sequential(s, cluster, mode, adjoint, kSeq, a, "sequential position kernel launch");
+    if (rc) return rc;
     const size_t n2 = (size_t)s->n * s->n;
     CKL(launch_q_to_probe(s->plan, t.Q.p, s->tmpc.p, s->twn.p, s->st), "q_to_probe");
     CK(cudaMemcpyAsync(rvol_out, t.V.p, sizeof(float) * n2 * s->nz, cudaMemcpyDeviceToHost, s->st));
@@ -664,8 +709,10 @@ int mset_forward_position(mset_session *s, int mode, int k, float row, float col
     rc = set_device(s);
     if (rc) return rc;
     s->step_k = -1;
+    bool cluster = false;
     rc = ensure_save(s, 1);
-    if (!rc) rc = refresh_tilt_table(s);
+    if (!rc) rc = seq_prepare(s, mode, 1, &cluster);
+    if (!rc && cluster) rc = seq_transmission(s, mode);
     if (rc) return rc;
     const int n = s->n;
     const size_t n2 = (size_t)n * n;
@@ -682,8 +729,8 @@ int mset_forward_position(mset_session *s, int mode, int k, float row, float col
     a.step_resi = s->step_resi.p;
     a.step_calc = s->step_calc.p;
     a.step_err = s->step_err.p;
-    const Plan &sp = seq_plan(s);
-    CKL(launch_positions(sp, mode, kREF, kStep, a, std::max(1, sp.cl), s->st), "STEP02 launch");
+    rc = launch_sequential(s, cluster, mode, kREF, kStep, a, "STEP02 launch");
+    if (rc) return rc;
     // the waves of field 0: slot 0 = psi0, slot s + 1 = wave after slab s
     std::vector<float2> resi(resi_out ? n2 : 0);
     if (resi_out)
@@ -743,6 +790,10 @@ int mset_adjoint_position(mset_session *s, int mode, int adjoint, const float *r
     }
     CK(s->step_grad.ensure(n2 * ns));
     CK(s->step_pos.ensure(2));
+    bool cluster = false;
+    rc = seq_prepare(s, mode, 1, &cluster);
+    if (!rc && cluster) rc = seq_transmission(s, mode);
+    if (rc) return rc;
     LaunchArgs a = base_args(s);
     a.step_phase = 2;
     a.step_k = s->step_k;
@@ -752,8 +803,8 @@ int mset_adjoint_position(mset_session *s, int mode, int adjoint, const float *r
     a.step_resi = s->step_resi.p;
     a.step_grad = s->step_grad.p;
     a.step_pos = s->step_pos.p;
-    const Plan &sp = seq_plan(s);
-    CKL(launch_positions(sp, mode, adjoint, kStep, a, std::max(1, sp.cl), s->st), "STEP03 launch");
+    rc = launch_sequential(s, cluster, mode, adjoint, kStep, a, "STEP03 launch");
+    if (rc) return rc;
     TiltBufs &t = s->tilts[0];
     std::vector<float2> g(grad_out ? n2 * ns : 0);
     if (grad_out)
@@ -785,7 +836,7 @@ int mset_set_sequential_split(mset_session *s, int on) {
 
 int mset_sequential_split(mset_session *s) {
     if (!s) return fail(MSET_E_ARG, "null session");
-    return (s->has_seq && s->seq_split) ? seq_plan(s).cl : 1;
+    return seq_on_cluster(s) ? s->seq->cl : 1;
 }
 
 int mset_read_state(mset_session *s, float *rvol_out, float *probe_out) {

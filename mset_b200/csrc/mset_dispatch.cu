@@ -11,8 +11,8 @@ namespace mset {
 // the autotuner may pick (at n = 256 the default stages the adjoint's
 // saved-wave rows by bulk copies: 1.443 s against 1.474 s per pass of 3 large
 // tilts on one B200).  At n = 128 the default is the three-phase shape; the
-// two-pass shape 128 after it has the layout of the sequential cluster
-// geometry 128c8 and serves the sequential entry points.
+// two-pass shape 128 after it has the layout of the sequential kernels and
+// serves the sequential entry points.
 #define MSET_GEOS(X) X(24) X(32) X(48) X(64) X(64v2) X(96) X(96v2) X(128t) X(128w) X(128) X(160) X(160v2) X(256s) X(256) X(256v2)
 #define X(N_) extern const GeoOps kGeo##N_;
 MSET_GEOS(X)
@@ -25,17 +25,38 @@ static const GeoOps *const kAllGeos[] = {
 };
 
 // the reference-semantics pass and the per-position steps walk one position
-// at a time through one field; these geometries split that field over a
-// thread-block cluster so one position uses several SMs
-#define MSET_SEQ_GEOS(X) X(128c8)
-#define X(N_) extern const GeoOps kSeqGeo##N_;
-MSET_SEQ_GEOS(X)
+// at a time: one field spread over the CTAs of a cluster (seq_kernel.cuh).
+// CTAs per field by measurement, microseconds per slab, forward and adjoint
+// (32 slabs of one plane, one B200):
+//   window   1 CTA   2       4       8       16
+//   24       1.90    2.30
+//   32       2.34    2.39    2.25
+//   48       6.03    4.50    3.69    3.19
+//   64               6.31    4.03    3.33
+//   96                       8.02    5.19    4.55
+//   128                              6.59    5.43
+//   160                              12.3    7.71
+//   256                              32.7    14.9
+// Small fields lose more to the exchanges than they gain; 128 keeps the 8
+// CTAs that mset_sequential_split documents.  The kernels before (one CTA per
+// field up to 160, 8 CTAs with remote loads and cluster barriers at 128) took
+// 8.4 us at 24 (24 slabs), 25.6 at 64 (24 slabs), 19.4 at 128 (64 slabs of two
+// planes) and 87 at 160 (95 slabs); these take 1.7, 3.1, 6.3 and 7.0 there.
+#define MSET_SEQ_FIELDS(X) X(24) X(32) X(48) X(64) X(96) X(128) X(160) X(256)
+#define X(N_) extern const SeqOps kSeqField##N_;
+MSET_SEQ_FIELDS(X)
 #undef X
-static const GeoOps *const kSeqGeos[] = {
-#define X(N_) &kSeqGeo##N_,
-    MSET_SEQ_GEOS(X)
+static const SeqOps *const kSeqFields[] = {
+#define X(N_) &kSeqField##N_,
+    MSET_SEQ_FIELDS(X)
 #undef X
 };
+
+const SeqOps *seq_ops_for(int n) {
+    for (const SeqOps *q : kSeqFields)
+        if (q->n == n) return q;
+    return nullptr;
+}
 
 static void fill_plan(const GeoOps *g, Plan *p) {
     p->n = g->n;
@@ -48,16 +69,6 @@ static void fill_plan(const GeoOps *g, Plan *p) {
     p->smem = g->smem;
     p->ctas_per_sm = 0;
     p->ops = g;
-}
-
-bool plan_seq_for(int n, Plan *p) {
-    for (const GeoOps *g : kSeqGeos)
-        if (g->n == n) {
-            fill_plan(g, p);
-            p->staged = 0;
-            return true;
-        }
-    return false;
 }
 
 static bool same_layout(const GeoOps *a, const GeoOps *b) { return a->r1 == b->r1 && a->ry1 == b->ry1; }

@@ -32,7 +32,8 @@ struct TiltDev {
     double *posdir;      // kBatch: [npos][2]
     double *err;         // [1] sum over positions and pixels of (A-M)^2
     float *inten;        // kSim: [npos][n][n] centred |Psi|^2
-    const float2 *T;     // [ns][n][n] precomputed transmission slabs, or null (computed from V)
+    const float2 *T;     // [ns][n][n] precomputed transmission slabs, or null (computed from V);
+                         // the sequential cluster kernels keep them up to date with V
     const unsigned short *ampb;  // [npos][n][n] scrambled ifftshift(I_meas) as BF16 bits, or null (use amp)
     int npos;
     int pad_;
@@ -64,6 +65,7 @@ struct LaunchArgs {
     float2 *step_grad;      // [ns][n][n] complex gradient i conj(T) conj(psi) chi (STEP03)
     float *step_pos;        // [2] updated scan coordinates (STEP03)
     double *step_err;       // [1] += sum over pixels of (A - M)^2 (STEP02; zeroed by the host)
+    double *seq_part;       // sequential cluster kernels: per-warp partial sums (seq_partials)
     unsigned *fault;        // [1] set by a kernel whose bounded wait gave up (may be null)
 };
 
@@ -80,12 +82,24 @@ struct GeoOps {
     int cl;  // CTAs per field (thread-block cluster size; 1: one CTA per position)
     size_t smem;
     int staged;  // the adjoint's saved-wave rows are staged in shared memory by bulk copies
+    int seq;     // the sequential modes are compiled for this shape
     int (*max_clusters)();  // clusters resident at once (cluster geometries)
     int (*positions)(int method, int adjoint, int mode, const LaunchArgs &a, int grid, cudaStream_t st);
     int (*prep_amp)(const float *meas_centred, float *amp_scr, long npos, cudaStream_t st);
     int (*prep_amp_bf16)(const float *meas_centred, unsigned short *i_scr, long npos, cudaStream_t st);
     int (*prep_prop)(const float *prop_centred, float2 *pscr, cudaStream_t st);
     int (*probe_q)(bool to_q, const float2 *in, float2 *out, const float2 *twn, cudaStream_t st);
+};
+
+// the sequential modes (kSeq, kStep) on one field over a cluster of cl CTAs
+// (seq_<N>.cu): window, residues of the scrambled layout in both dimensions,
+// warps of the whole cluster
+struct SeqOps {
+    int n, r1;
+    int cl;
+    int warps;
+    bool (*fits)();  // the device can hold the cluster
+    int (*positions)(int method, int adjoint, int mode, const LaunchArgs &a, cudaStream_t st);
 };
 
 // host-side launchers (return cudaError_t as int)
@@ -104,10 +118,10 @@ bool plan_for(int n, Plan *p, int variant = 0);
 // the first geometry of window n whose scrambled layouts have r1 x residues
 // and ry1 y residues
 bool plan_for_layout(int n, int r1, int ry1, Plan *p);
-// the cluster geometry of window n for the sequential modes (kSeq, kStep),
-// when one is compiled (the sessions of those modes use the one-CTA shape with
-// its scrambled layouts, plan_for_layout)
-bool plan_seq_for(int n, Plan *p);
+// the sequential modes' kernels of window n (null: none compiled); the sessions
+// of those modes use the one-CTA shape with their scrambled layouts
+// (plan_for_layout)
+const SeqOps *seq_ops_for(int n);
 int plan_variants(int n);
 int launch_positions(const Plan &pl, int method, int adjoint, int mode, const LaunchArgs &a, int grid,
                      cudaStream_t st);

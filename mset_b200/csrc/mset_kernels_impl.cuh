@@ -1110,32 +1110,20 @@ int geo_max_clusters() {
     }
 }
 
-template <class G>
+// SEQ: the sequential modes on one CTA (or the batched cluster) per field too,
+// for sessions that turn the split over a cluster off
+template <class G, bool SEQ>
 int geo_positions(int method, int adjoint, int mode, const LaunchArgs &a, int grid, cudaStream_t st) {
     if (mode == kErr || mode == kSim) adjoint = kREF;
 #define MSET_L(M, A, MO) \
     if (method == M && adjoint == A && mode == MO) return launch_one<G, M, A, MO>(a, grid, st);
-    MSET_L(kMSET, kREF, kSeq) MSET_L(kMSET, kREF, kBatch) MSET_L(kMSET, kEXACT, kSeq) MSET_L(kMSET, kEXACT, kBatch)
-    MSET_L(kSSET, kREF, kSeq) MSET_L(kSSET, kREF, kBatch) MSET_L(kSSET, kEXACT, kSeq) MSET_L(kSSET, kEXACT, kBatch)
+    MSET_L(kMSET, kREF, kBatch) MSET_L(kMSET, kEXACT, kBatch) MSET_L(kSSET, kREF, kBatch) MSET_L(kSSET, kEXACT, kBatch)
     MSET_L(kMSET, kREF, kErr) MSET_L(kSSET, kREF, kErr) MSET_L(kMSET, kREF, kSim) MSET_L(kSSET, kREF, kSim)
     MSET_L(kMSET, kREF, kBatchCk) MSET_L(kMSET, kEXACT, kBatchCk)
-    MSET_L(kMSET, kREF, kStep) MSET_L(kMSET, kEXACT, kStep) MSET_L(kSSET, kREF, kStep) MSET_L(kSSET, kEXACT, kStep)
-#undef MSET_L
-    return (int)cudaErrorInvalidValue;
-}
-
-// (a geometry whose batched queue is never launched: one cluster per call)
-inline int geo_no_clusters() { return 0; }
-
-// the modes that walk one position at a time through one field: the
-// reference-semantics pass (kSeq) and the per-position steps (kStep); a
-// geometry compiled for these alone splits that one field over a cluster
-template <class G>
-int geo_positions_seq(int method, int adjoint, int mode, const LaunchArgs &a, int grid, cudaStream_t st) {
-#define MSET_L(M, A, MO) \
-    if (method == M && adjoint == A && mode == MO) return launch_one<G, M, A, MO>(a, grid, st);
-    MSET_L(kMSET, kREF, kSeq) MSET_L(kMSET, kEXACT, kSeq) MSET_L(kSSET, kREF, kSeq) MSET_L(kSSET, kEXACT, kSeq)
-    MSET_L(kMSET, kREF, kStep) MSET_L(kMSET, kEXACT, kStep) MSET_L(kSSET, kREF, kStep) MSET_L(kSSET, kEXACT, kStep)
+    if constexpr (SEQ) {
+        MSET_L(kMSET, kREF, kSeq) MSET_L(kMSET, kEXACT, kSeq) MSET_L(kSSET, kREF, kSeq) MSET_L(kSSET, kEXACT, kSeq)
+        MSET_L(kMSET, kREF, kStep) MSET_L(kMSET, kEXACT, kStep) MSET_L(kSSET, kREF, kStep) MSET_L(kSSET, kEXACT, kStep)
+    }
 #undef MSET_L
     return (int)cudaErrorInvalidValue;
 }
@@ -1167,46 +1155,25 @@ int geo_probe_q(bool to_q, const float2 *in, float2 *out, const float2 *twn, cud
 
 }  // namespace mset
 
-// one translation unit per window size defines its table entry
-#define MSET_DEFINE_GEO(N_, R1_, NT_, MINB_) MSET_DEFINE_GEO_T(N_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>))
+// one translation unit per window size defines its table entry; _SEQ: with
+// the sequential modes on this shape
+#define MSET_DEFINE_GEO(N_, R1_, NT_, MINB_) MSET_DEFINE_GEO_T(N_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), false)
+#define MSET_DEFINE_GEO_SEQ(N_, R1_, NT_, MINB_) MSET_DEFINE_GEO_T(N_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), true)
 // another thread / register shape of the same window (same R1, so the same
 // scrambled layouts): a choice for the autotuner, table entry kGeo<NAME_>
 #define MSET_DEFINE_GEO_VARIANT(NAME_, N_, R1_, NT_, MINB_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>))
-// the same window and thread shape with the adjoint's saved-wave rows staged
-// in shared memory by bulk copies (StageCfg)
-#define MSET_DEFINE_GEO_STAGED(NAME_, N_, R1_, NT_, MINB_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_, true>))
-// the sequential modes only (geo_positions_seq), with one field split by rows
-// over a cluster of CL_ CTAs: table entry kSeqGeo<NAME_>
-#define MSET_DEFINE_SEQ_GEO_CL(NAME_, N_, R1_, NT_, CL_)                                \
-    namespace mset {                                                                   \
-    using SeqGeo##NAME_ = GeoCl<N_, R1_, NT_, CL_>;                                    \
-    extern const GeoOps kSeqGeo##NAME_ = {N_,                                          \
-                                          R1_,                                         \
-                                          SeqGeo##NAME_::RY1,                          \
-                                          SeqGeo##NAME_::NT,                           \
-                                          SeqGeo##NAME_::CL,                           \
-                                          smem_bytes<SeqGeo##NAME_>(),                 \
-                                          0,                                           \
-                                          &geo_no_clusters,                            \
-                                          &geo_positions_seq<SeqGeo##NAME_>,           \
-                                          &geo_prep_amp<SeqGeo##NAME_>,                \
-                                          &geo_prep_amp_bf16<SeqGeo##NAME_>,           \
-                                          &geo_prep_prop<SeqGeo##NAME_>,               \
-                                          &geo_probe_q<SeqGeo##NAME_>};                \
-    }
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), false)
 // a field split by rows over a cluster of CL_ CTAs
-#define MSET_DEFINE_GEO_CL(N_, R1_, NT_, CL_) MSET_DEFINE_GEO_T(N_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_>))
+#define MSET_DEFINE_GEO_CL(N_, R1_, NT_, CL_) MSET_DEFINE_GEO_T(N_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_>), false)
 // the same with the adjoint's saved-wave rows staged by bulk copies (StageCfg)
 #define MSET_DEFINE_GEO_CL_STAGED(NAME_, N_, R1_, NT_, CL_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, 1, true>))
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, 1, true>), true)
 #define MSET_DEFINE_GEO_CL_VARIANT(NAME_, N_, R1_, NT_, CL_, MINB_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, MINB_>))
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, MINB_>), false)
 // the three-phase shape of the 128 x 128 window (Geo3; WIDE_: 16-byte phase-2 accesses)
-#define MSET_DEFINE_GEO3(NAME_, WIDE_) MSET_DEFINE_GEO_T(NAME_, 128, 8, (Geo3<1, WIDE_>))
+#define MSET_DEFINE_GEO3(NAME_, WIDE_) MSET_DEFINE_GEO_T(NAME_, 128, 8, (Geo3<1, WIDE_>), false)
 #define MSET_UNPAREN(...) __VA_ARGS__
-#define MSET_DEFINE_GEO_T(NAME_, N_, R1_, GT_)                                         \
+#define MSET_DEFINE_GEO_T(NAME_, N_, R1_, GT_, SEQ_)                                   \
     namespace mset {                                                                   \
     using Geo##NAME_ = MSET_UNPAREN GT_;                                               \
     extern const GeoOps kGeo##NAME_ = {N_,                                             \
@@ -1216,8 +1183,9 @@ int geo_probe_q(bool to_q, const float2 *in, float2 *out, const float2 *twn, cud
                                        Geo##NAME_::CL,                                 \
                                        smem_bytes<Geo##NAME_>(),                       \
                                        StageCfg<Geo##NAME_>::kOn ? 1 : 0,              \
+                                       SEQ_ ? 1 : 0,                                   \
                                        &geo_max_clusters<Geo##NAME_>,                  \
-                                       &geo_positions<Geo##NAME_>,                     \
+                                       &geo_positions<Geo##NAME_, SEQ_>,               \
                                        &geo_prep_amp<Geo##NAME_>,                      \
                                        &geo_prep_amp_bf16<Geo##NAME_>,                 \
                                        &geo_prep_prop<Geo##NAME_>,                     \

@@ -196,7 +196,7 @@ class Session:
 
     def set_sequential_split(self, on: bool) -> None:
         """split one position's field over a thread-block cluster in run() and
-        the per-position steps (default on where compiled, n = 128)"""
+        the per-position steps (default on)"""
         check("mset_set_sequential_split", self._lib.mset_set_sequential_split(self._h, int(bool(on))))
 
     def sequential_split(self) -> int:
