@@ -260,9 +260,9 @@ int mset_batch_read_gradient(mset_session *s, double *grad, double *probe, doubl
  * (up to 4 x SMs x resident CTAs) for every shape whose saved-wave storage fits
  * mem_budget_bytes (0: no limit) and keeps the fastest, or among shapes within
  * 1% of it the one using less memory.  Shape = kernel thread shape (two or
- * three compiled shapes for 64, 96, 128, 160 and 256: threads per CTA and the
- * register budget that goes with them, row padding, or the saved waves staged
- * by bulk copies) x persistent CTAs (SMs x CTAs per
+ * three compiled shapes for 48, 64, 96, 128, 160 and 256: threads per CTA and
+ * the register budget that goes with them, row padding, or the saved waves
+ * staged by bulk copies; the untuned default is chosen by positions per SM) x persistent CTAs (SMs x CTAs per
  * SM, i.e. positions in flight) x checkpoint interval k in {0, 2, 4, 8, 16}
  * (k < slabs; k = 0 keeps every wave).  The choice stays with the session
  * (mset_batch_set_checkpoint overrides k).  MSET_E_NOMEM when no shape fits. */

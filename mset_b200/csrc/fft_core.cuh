@@ -1,8 +1,9 @@
 // fft_core.cuh -- shared-memory 2D FFT building blocks for sm_100a.
 //
 // An N x N complex64 field lives in one CTA's shared memory, row stride
-// S = N + N/R1 (one pad element after every R1 elements along x, which makes
-// every pass below free of bank conflicts).  A 1D transform of length
+// S = N + N/R1, one pad element after every R1 elements along x (R1 = R2 = 8:
+// no pads, each group of 8 rotated by its index instead), which makes every
+// pass below free of bank conflicts at R1 = 16 and at 64 x 64.  A 1D transform of length
 // N = R1*R2 is two register passes:
 //
 //   pass A (per n1, R2 points at x = n1 + R1*j):   R2-point DFT + twiddle
@@ -271,8 +272,31 @@ struct Geo {
     static constexpr bool THREE = false;  // the three-phase shape (Geo3)
     static constexpr int CB = R1;         // points of a column-pass-B task
     static constexpr int RY1 = R1;        // the y dimension's factors (the x ones here)
+    // Two pad-separated groups of 8 columns share a bank, so at R1 = 8 a
+    // half-warp's 16 adjacent columns of a column pass would take two
+    // wavefronts.  At 8 x 8 the elements of group g are rotated by g inside the
+    // group and the row stride is 8 mod 16: row pass A (8 elements of one group
+    // of two rows), row pass B (element j of 8 groups of two rows) and the
+    // column passes (two adjacent groups) each touch 16 different bank pairs.
+    static constexpr bool ROT = R1 == 8 && R2 == 8;
     static_assert(R1 * R2 == N, "N must equal R1*R2");
-    __device__ __forceinline__ static int px(int x) { return x + x / R1; }
+    __device__ __forceinline__ static int px(int x) {
+        if constexpr (ROT) return (x & ~7) + ((x + (x >> 3)) & 7);
+        else return x + x / R1;
+    }
+    // position in a row of x = n1 + R1 j: xa0(n1) + xa(n1, j), and of x = j +
+    // R1 k2: xb0(k2) + xb(k2, j) (constant offsets from one address unless
+    // rotated)
+    __device__ __forceinline__ static int xa0(int n1) { return ROT ? 0 : n1; }
+    __device__ __forceinline__ static int xa(int n1, int j) {
+        if constexpr (ROT) return 8 * j + ((n1 + j) & 7);
+        else return (R1 + 1) * j;
+    }
+    __device__ __forceinline__ static int xb0(int k2) { return ROT ? 8 * k2 : (R1 + 1) * k2; }
+    __device__ __forceinline__ static int xb(int k2, int j) {
+        if constexpr (ROT) return (j + k2) & 7;
+        else return j;
+    }
     __device__ __forceinline__ static int at(int y, int x) { return y * S + px(x); }
     // scrambled location -> frequency index (both dimensions)
     __host__ __device__ __forceinline__ static int scr(int L) { return L / R1 + R2 * (L % R1); }
@@ -282,6 +306,31 @@ struct Geo {
     // row of the field held at local row l (yb = ybase(), read once per pass)
     __device__ __forceinline__ static int ybase() { return 0; }
     __device__ __forceinline__ static int gy(int, int l) { return l; }
+    // Order of the kernel's own per-slab fields in global memory (transmission,
+    // saved waves): natural rows, or at R1 = 8, where the 8 lanes of a row
+    // would touch half a 128-byte line, the order in which row pass A's lanes
+    // take them: per 4 rows and j, the 32 lanes' elements side by side (half
+    // the L1 wavefronts of these accesses).  Element x = n1 + R1 j of row y is
+    // at grow(y) GR + n1 + GJ j.
+    static constexpr bool LANES = R1 == 8;
+    static constexpr int GJ = LANES ? 32 : R1, GR = LANES ? 8 : N;
+    __device__ __forceinline__ static int grow(int y) {
+        if constexpr (LANES) return (y >> 2) * (R2 * 4) + (y & 3);
+        else return y;
+    }
+    // row and column of element l of that order (LANES)
+    __device__ __forceinline__ static void gpos(int l, int &y, int &x) {
+        const int blk = (l >> 5) / R2, j = (l >> 5) % R2;
+        y = blk * 4 + ((l >> 3) & 3);
+        x = (l & 7) + R1 * j;
+    }
+    // byte offset of the k-th 128-byte line of row y's share (L1 hints)
+    static constexpr int kRow = (int)sizeof(float2) * N, kLPR = (kRow + 127) / 128;
+    __device__ __forceinline__ static size_t line(int y, int k) {
+        if constexpr (LANES)
+            return (y >> 2) * (R2 * 256) + min(((y & 3) * kLPR + k) * 128, R2 * 256 - (int)sizeof(float2));
+        else return (size_t)y * kRow + min(k * 128, kRow - (int)sizeof(float2));
+    }
 };
 
 // A field too large for one SM's shared memory, split by rows over a
@@ -361,6 +410,18 @@ struct Geo3 {
     __device__ __forceinline__ static int rank() { return 0; }
     __device__ __forceinline__ static int ybase() { return 0; }
     __device__ __forceinline__ static int gy(int, int l) { return l; }
+    // lane order of the per-slab fields (see Geo): the 4 rows of a phase-1 warp
+    // iteration, {2w, 2w + 1} + {0, 32} + 64 it, make one block
+    static constexpr bool LANES = true;
+    static constexpr int GJ = 32, GR = 8;
+    __device__ __forceinline__ static int grow(int y) {
+        return ((y >> 6) * 16 + ((y & 31) >> 1)) * (R2 * 4) + (y & 1) + ((y >> 4) & 2);
+    }
+    __device__ __forceinline__ static void gpos(int l, int &y, int &x) {
+        const int blk = (l >> 5) / R2, j = (l >> 5) % R2;
+        y = (blk >> 4) * 64 + ((l >> 4) & 1) * 32 + (blk & 15) * 2 + ((l >> 3) & 1);
+        x = (l & 7) + R1 * j;
+    }
 };
 
 // twiddle W_N^{n1 k2} with sign (table holds e^{-2 pi i m/N} as [k2][n1])
@@ -543,10 +604,10 @@ __device__ __forceinline__ void row_passA_pf(float2 *buf, const float2 *tw, Pf &
             } else {
                 pf(y, n1, pre);
             }
-            float2 *row = buf + (yl0 + tau / R1) * G::S + n1;
+            float2 *row = buf + (yl0 + tau / R1) * G::S + G::xa0(n1);
             float2 v[R2];
 #pragma unroll
-            for (int j = 0; j < R2; ++j) v[j] = row[(R1 + 1) * j];
+            for (int j = 0; j < R2; ++j) v[j] = row[G::xa(n1, j)];
             auto twi = [&](int k2, auto sg) -> float2 {
                 constexpr int SG = decltype(sg)::value;
                 if constexpr (kTwReg) return SG < 0 ? twr[k2] : cconj(twr[k2]);
@@ -573,7 +634,7 @@ __device__ __forceinline__ void row_passA_pf(float2 *buf, const float2 *tw, Pf &
                 for (int k2 = 1; k2 < R2; ++k2) v[k2] = cmul(v[k2], twi(k2, std::integral_constant<int, OUT>{}));
             }
 #pragma unroll
-            for (int j = 0; j < R2; ++j) row[(R1 + 1) * j] = v[j];
+            for (int j = 0; j < R2; ++j) row[G::xa(n1, j)] = v[j];
             if constexpr (ahead) pre = nxt;
         }
     }
@@ -609,13 +670,13 @@ __device__ __forceinline__ void row_passB(float2 *buf) {
 #pragma unroll 1
     for (int tau = O::lane(); tau < TASKS; tau += 32) {
         const int k2 = tau % R2, y = y0 + tau / R2;
-        float2 *p = buf + y * G::S + (R1 + 1) * k2;
+        float2 *p = buf + y * G::S + G::xb0(k2);
         float2 v[R1];
 #pragma unroll
-        for (int j = 0; j < R1; ++j) v[j] = p[j];
+        for (int j = 0; j < R1; ++j) v[j] = p[G::xb(k2, j)];
         DFT<R1, SG>::run(v);
 #pragma unroll
-        for (int j = 0; j < R1; ++j) p[j] = v[j];
+        for (int j = 0; j < R1; ++j) p[G::xb(k2, j)] = v[j];
     }
 }
 

@@ -1,3 +1,3 @@
-// kernels for 128 x 128 windows
+// kernels for 128 x 128 windows in the sequential sessions' layout
 #include "mset_kernels_impl.cuh"
-MSET_DEFINE_GEO_SEQ(128, 16, 512, 1)
+MSET_DEFINE_GEO_SEQ_ONLY(128, 128, 16, 512, 1)

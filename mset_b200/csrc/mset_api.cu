@@ -106,6 +106,7 @@ struct mset_session {
     float sigma = 0, dz = 0, step[3] = {0, 0, 0};
     int nsx = 0, nsy = 0;
     Plan plan{};
+    Plan plan_default{};  // the shape the session was set up with
     // sequential modes (kSeq, kStep): the window's kernels on a cluster per
     // field (seq_split: in use; kernels of one CTA per field always are)
     const SeqOps *seq = nullptr;
@@ -211,22 +212,22 @@ int scrambled_freq(int L, int n, int r) { return L / r + (n / r) * (L % r); }
 // per-position steps), whose one-CTA shape takes the scrambled layouts of the
 // window's cluster geometry for that pass when one is compiled
 int ensure_geometry(mset_session *s, int n, int nz, int b, float sigma, float dz, const float *prop,
-                    bool sequential) {
+                    bool sequential, long positions) {
     if (n <= 1 || nz <= 0 || b <= 0) return fail(MSET_E_ARG, "invalid sizes n=%d nz=%d slice_binning=%d", n, nz, b);
     Plan pl;
-    if (!plan_for(n, &pl))
+    if (!plan_for(n, positions, s->sms, &pl))
         return fail(MSET_E_UNSUPPORTED,
                     "window size %d has no compiled kernel (supported: 24, 32, 48, 64, 96, 128, 160, 256)", n);
     if (b > nz) b = nz;  // STEP00_INIT.m:126-128
     const SeqOps *sq = sequential ? seq_ops_for(n) : nullptr;
-    if (sq && !sq->fits()) sq = nullptr;
-    if (sq && (sq->r1 != pl.r1 || sq->r1 != pl.ry1)) {
-        Plan alt;
-        if (plan_for_layout(n, sq->r1, sq->r1, &alt)) pl = alt;
-        else sq = nullptr;
+    if (sequential) {
+        Plan one;
+        if (plan_for_seq(n, &one)) pl = one;
+        if (sq && (!sq->fits() || sq->r1 != pl.r1 || sq->r1 != pl.ry1)) sq = nullptr;
     }
     if (pl.cl > 1) pl.max_clusters = pl.ops->max_clusters();
     s->plan = pl;
+    s->plan_default = pl;
     s->seq = sq;
     s->n = n;
     s->nz = nz;
@@ -577,7 +578,8 @@ static int upload_impl(mset_session *s, const mset_upload_args *a, const float *
     s->batch = false;
     s->step_k = -1;
     s->ckpt = 0;  // the sequential kernels keep every slab's wave
-    rc = ensure_geometry(s, a->n, a->nz, a->slice_binning, a->sigma, a->potential_pixelsize, a->prop2D, true);
+    rc = ensure_geometry(s, a->n, a->nz, a->slice_binning, a->sigma, a->potential_pixelsize, a->prop2D, true,
+                         a->num_scan_pos);
     if (rc) return rc;
     s->step[0] = a->step_size[0];
     s->step[1] = a->step_size[1];
@@ -896,7 +898,9 @@ int mset_batch_setup(mset_session *s, const mset_batch_args *a) {
     int rc = set_device(s);
     if (rc) return rc;
     s->ready = false;
-    rc = ensure_geometry(s, a->n, a->nz, a->slice_binning, a->sigma, a->potential_pixelsize, a->prop2D, false);
+    long positions = 0;
+    for (int j = 0; j < a->ntilts; ++j) positions += std::max(0, a->npos[j]);
+    rc = ensure_geometry(s, a->n, a->nz, a->slice_binning, a->sigma, a->potential_pixelsize, a->prop2D, false, positions);
     if (rc) return rc;
     s->method = a->method;
     s->adjoint = a->adjoint;
@@ -994,7 +998,7 @@ static int batch_zero(mset_session *s) {
 static int batch_transmission_enqueue(mset_session *s) {
     const int nsg = s->method == MSET_MODE_SSET ? 1 : s->ns;
     const int b = s->method == MSET_MODE_SSET ? s->nz : s->b;
-    CKL(launch_transmission(s->d_tilts.p, (int)s->tilts.size(), s->n, s->nz, b, nsg, s->sigma * s->dz, s->st),
+    CKL(s->plan.ops->transmission(s->d_tilts.p, (int)s->tilts.size(), s->nz, b, nsg, s->sigma * s->dz, s->st),
         "transmission");
     return 0;
 }
@@ -1438,7 +1442,7 @@ static int record_phase(mset_session *s, int phase, bool with_tv = true, bool wi
         CK(cudaMemsetAsync(t.qacc.p, 0, sizeof(double) * n2 * 2, s->st));
     }
     CK(cudaMemsetAsync(s->err.p, 0, sizeof(double) * J, s->st));
-    CKL(launch_transmission(s->d_tilts.p, J, n, s->nz, bvox, nsg, s->sigma * s->dz, s->st), "transmission");
+    CKL(s->plan.ops->transmission(s->d_tilts.p, J, s->nz, bvox, nsg, s->sigma * s->dz, s->st), "transmission");
     CK(cudaMemsetAsync(s->counter.p, 0, sizeof(unsigned), s->st));
     {
         LaunchArgs la = base_args(s);
@@ -1556,7 +1560,7 @@ static int record_error_phase(mset_session *s) {
         CKL(vol_pad(s->gvol.p, s->tilts[j].V.p, s->nv1, s->nv2, s->nv3, n, s->st), "pad");
     }
     CK(cudaMemsetAsync(s->err.p, 0, sizeof(double) * J, s->st));
-    CKL(launch_transmission(s->d_tilts.p, J, n, s->nz, bvox, nsg, s->sigma * s->dz, s->st), "transmission");
+    CKL(s->plan.ops->transmission(s->d_tilts.p, J, s->nz, bvox, nsg, s->sigma * s->dz, s->st), "transmission");
     CK(cudaMemsetAsync(s->counter.p, 0, sizeof(unsigned), s->st));
     LaunchArgs la = base_args(s);
     CKL(launch_positions(s->plan, s->method, kREF, kErr, la, s->grid_cache, s->st), "error pass");
@@ -1822,7 +1826,7 @@ int tune_session(mset_session *s, double budget, mset_tune_result *out) {
     int occ_max = 1;
     for (int v = 0; v < plan_variants(s->n); ++v) {
         Plan pl;
-        if (plan_for(s->n, &pl, v)) {
+        if (plan_variant(s->plan_default, v, &pl)) {
             s->plan = pl;
             occ_max = std::max(occ_max, occupancy_limit(s));
         }
@@ -1838,7 +1842,7 @@ int tune_session(mset_session *s, double budget, mset_tune_result *out) {
     const int tuned_in = s->tuned_grid;
     for (int v = 0; v < plan_variants(s->n); ++v) {
         Plan pl;
-        if (!plan_for(s->n, &pl, v)) continue;
+        if (!plan_variant(s->plan_default, v, &pl)) continue;
         if (pl.cl > 1) pl.max_clusters = pl.ops->max_clusters();
         s->plan = pl;
         const int occ = occupancy_limit(s);
@@ -2052,7 +2056,7 @@ int mset_batch_set_variant(mset_session *s, int variant) {
     int rc = batch_ok(s);
     if (rc) return rc;
     Plan pl;
-    if (variant < 0 || !plan_for(s->n, &pl, variant))
+    if (variant < 0 || !plan_variant(s->plan_default, variant, &pl))
         return fail(MSET_E_ARG, "window %d has %d kernel shapes, not %d", s->n, plan_variants(s->n), variant + 1);
     if (pl.cl > 1) pl.max_clusters = pl.ops->max_clusters();
     s->plan = pl;

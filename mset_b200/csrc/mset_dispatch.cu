@@ -1,25 +1,48 @@
 // mset_dispatch.cu -- window-size dispatch and the size-independent
 // kernels of the batched update.
 #include <algorithm>
+#include <cmath>
 #include "mset_kernels.cuh"
 
 
 namespace mset {
 
-// every compiled geometry; the first entry of a window size is its default,
-// the others with the same scrambled layouts are alternative thread shapes
-// the autotuner may pick (at n = 256 the default stages the adjoint's
-// saved-wave rows by bulk copies: 1.443 s against 1.474 s per pass of 3 large
-// tilts on one B200).  At n = 128 the default is the three-phase shape; the
-// two-pass shape 128 after it has the layout of the sequential kernels and
-// serves the sequential entry points.
-#define MSET_GEOS(X) X(24) X(32) X(48) X(64) X(64v2) X(96) X(96v2) X(128t) X(128w) X(128) X(160) X(160v2) X(256s) X(256) X(256v2)
-#define X(N_) extern const GeoOps kGeo##N_;
+// Every compiled geometry.  The default shape of a batched session is the
+// first entry of its window whose range (lo, hi] holds its positions per SM
+// (entries with an empty range are the autotuner's alternatives); the shapes
+// with the same scrambled layouts are the session's variants.  The lines, by
+// measurement (one B200, microseconds per pass of P positions):
+//  24, 32  one shape (192 threads at 24: 81 us at P = 148, 648 at 3000, 24
+//          slabs; 64 threads took 138 and 805)
+//  48      192 threads with 128 registers x 2 CTAs up to 2 positions per SM
+//          (244 against 271 at P = 296), x 4 above (1286 against 1517 at 2000)
+//  64      256 threads x 2 CTAs up to 6 positions per SM (349 against 411 at P =
+//          296, 804 against 846 at 740), 128 x 4 above (9645 against 10574 at P
+//          = 8000, 32 slabs)
+//  96      384 threads x 2 CTAs (80 registers; 3600 at P = 1184, 32 slabs,
+//          against 4380 with one CTA and 128 registers); one CTA up to one
+//          position per SM (584 against 635 at P = 148)
+//  128     the three-phase shape; the two-pass one serves the sequential
+//          sessions
+//  256     the saved-wave rows staged by bulk copies (1.443 s against 1.474 s
+//          per pass of 3 large tilts)
+// At 24, 32, 64 and 128 the transmission and the saved waves are kept in the
+// kernel's lane order (Geo::LANES): 172.0 -> 165.2 ns per slab of a position at
+// 128, 44.1 -> 42.4 at 64; at 64 the rotated rows (Geo::ROT) gave 52.3 -> 44.1.
+struct GeoEntry {
+    const GeoOps *g;
+    float lo, hi;
+};
+#define MSET_GEOS(X)                                                                                          \
+    X(24, 0, INFINITY) X(32, 0, INFINITY) X(48a, 2, INFINITY) X(48, 0, 2) X(64p, 6, INFINITY) X(64, 0, 6) \
+    X(96a, 1, INFINITY) X(96, 0, 1) X(128t, 0, INFINITY) X(128w, 0, 0) X(128, 0, 0) X(160, 0, INFINITY)       \
+    X(160v2, 0, 0) X(256s, 0, INFINITY) X(256, 0, 0) X(256v2, 0, 0)
+#define X(N_, LO_, HI_) extern const GeoOps kGeo##N_;
 MSET_GEOS(X)
 #undef X
 
-static const GeoOps *const kAllGeos[] = {
-#define X(N_) &kGeo##N_,
+static const GeoEntry kAllGeos[] = {
+#define X(N_, LO_, HI_) {&kGeo##N_, LO_, HI_},
     MSET_GEOS(X)
 #undef X
 };
@@ -71,41 +94,52 @@ static void fill_plan(const GeoOps *g, Plan *p) {
     p->ops = g;
 }
 
-static bool same_layout(const GeoOps *a, const GeoOps *b) { return a->r1 == b->r1 && a->ry1 == b->ry1; }
-
-static const GeoOps *default_geo(int n) {
-    for (const GeoOps *g : kAllGeos)
-        if (g->n == n) return g;
-    return nullptr;
+static bool same_layout(const GeoOps *a, const GeoOps *b) {
+    return a->n == b->n && a->r1 == b->r1 && a->ry1 == b->ry1;
 }
 
-// the shapes of window n with the default's scrambled layouts, default first
-static const GeoOps *find_geo(int n, int variant) {
-    const GeoOps *d = default_geo(n);
-    if (!d) return nullptr;
-    for (const GeoOps *g : kAllGeos)
-        if (g->n == n && same_layout(g, d) && variant-- == 0) return g;
-    return nullptr;
+bool plan_for(int n, long positions, int sms, Plan *p) {
+    const float per_sm = (float)positions / (float)(sms > 0 ? sms : 1);
+    const GeoOps *first = nullptr;
+    for (const GeoEntry &e : kAllGeos) {
+        if (e.g->n != n) continue;
+        if (!first) first = e.g;
+        if (e.lo < per_sm && per_sm <= e.hi) {
+            fill_plan(e.g, p);
+            return true;
+        }
+    }
+    if (first) fill_plan(first, p);  // no positions yet
+    return first != nullptr;
+}
+
+bool plan_for_seq(int n, Plan *p) {
+    for (const GeoEntry &e : kAllGeos)
+        if (e.g->n == n && e.g->seq) {
+            fill_plan(e.g, p);
+            return true;
+        }
+    return false;
 }
 
 int plan_variants(int n) {
-    const GeoOps *d = default_geo(n);
+    const GeoOps *d = nullptr;
     int c = 0;
-    for (const GeoOps *g : kAllGeos) c += d && g->n == n && same_layout(g, d);
+    for (const GeoEntry &e : kAllGeos) {
+        if (e.g->n == n && !d) d = e.g;
+        c += d && e.g->batch && same_layout(e.g, d);
+    }
     return c;
 }
 
-bool plan_for(int n, Plan *p, int variant) {
-    const GeoOps *g = find_geo(n, variant);
-    if (!g) return false;
-    fill_plan(g, p);
-    return true;
-}
-
-bool plan_for_layout(int n, int r1, int ry1, Plan *p) {
-    for (const GeoOps *g : kAllGeos)
-        if (g->n == n && g->r1 == r1 && g->ry1 == ry1) {
-            fill_plan(g, p);
+bool plan_variant(const Plan &base, int variant, Plan *p) {
+    if (variant == 0) {
+        fill_plan(base.ops, p);
+        return true;
+    }
+    for (const GeoEntry &e : kAllGeos)
+        if (e.g != base.ops && e.g->batch && same_layout(e.g, base.ops) && --variant == 0) {
+            fill_plan(e.g, p);
             return true;
         }
     return false;

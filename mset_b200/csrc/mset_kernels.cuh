@@ -83,12 +83,15 @@ struct GeoOps {
     size_t smem;
     int staged;  // the adjoint's saved-wave rows are staged in shared memory by bulk copies
     int seq;     // the sequential modes are compiled for this shape
+    int batch;   // the batched modes are
     int (*max_clusters)();  // clusters resident at once (cluster geometries)
     int (*positions)(int method, int adjoint, int mode, const LaunchArgs &a, int grid, cudaStream_t st);
     int (*prep_amp)(const float *meas_centred, float *amp_scr, long npos, cudaStream_t st);
     int (*prep_amp_bf16)(const float *meas_centred, unsigned short *i_scr, long npos, cudaStream_t st);
     int (*prep_prop)(const float *prop_centred, float2 *pscr, cudaStream_t st);
     int (*probe_q)(bool to_q, const float2 *in, float2 *out, const float2 *twn, cudaStream_t st);
+    // transmission slabs in the order the shape's kernels read them
+    int (*transmission)(const TiltDev *tilts_dev, int ntilts, int nz, int b, int ns, float sdz, cudaStream_t st);
 };
 
 // the sequential modes (kSeq, kStep) on one field over a cluster of cl CTAs
@@ -112,16 +115,19 @@ struct Plan {
     int ctas_per_sm;
     const GeoOps *ops;
 };
-// geometry `variant` (0: default) of window size n; plan_variants(n) of them
-// exist, all with the default's scrambled layouts
-bool plan_for(int n, Plan *p, int variant = 0);
-// the first geometry of window n whose scrambled layouts have r1 x residues
-// and ry1 y residues
-bool plan_for_layout(int n, int r1, int ry1, Plan *p);
+// the default shape of a batched session with this many positions in all its
+// tilts; false: the window has no compiled kernels
+bool plan_for(int n, long positions, int sms, Plan *p);
+// the shape of a sequential session: the one with the sequential modes on one
+// CTA per field (false: the window has none)
+bool plan_for_seq(int n, Plan *p);
+// shapes that share the scrambled layouts of `base`, base itself first
+bool plan_variant(const Plan &base, int variant, Plan *p);
 // the sequential modes' kernels of window n (null: none compiled); the sessions
-// of those modes use the one-CTA shape with their scrambled layouts
-// (plan_for_layout)
+// of those modes use the one-CTA shape of plan_for_seq, which has their
+// scrambled layouts
 const SeqOps *seq_ops_for(int n);
+// shapes with the layout of the window's first one
 int plan_variants(int n);
 int launch_positions(const Plan &pl, int method, int adjoint, int mode, const LaunchArgs &a, int grid,
                      cudaStream_t st);
@@ -135,6 +141,7 @@ int launch_q_to_probe(const Plan &pl, const float2 *q, float2 *probe, const floa
 void set_last_error(const char *msg);
 
 int launch_apply_probe_pos(const TiltDev *tilts_host, int ntilts, int n, float step1, float step2, cudaStream_t st);
+// transmission slabs in natural order (y, x)
 int launch_transmission(const TiltDev *tilts_dev, int ntilts, int n, int nz, int b, int ns, float sdz,
                         cudaStream_t st);
 int launch_apply_batch(int n, int nz, int b, int ns, int method, float step0, float step1, float step2,

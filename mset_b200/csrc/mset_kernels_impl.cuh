@@ -15,6 +15,7 @@
 // (the batched method).  kErr is run_error_mset/_sset (mset.cu:557-810).
 #pragma once
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <utility>
 #include "fft_core.cuh"
 #include "mset_kernels.cuh"
@@ -119,8 +120,7 @@ struct L1Rows {
     __device__ __forceinline__ void operator()(int y, int k) const {
         const char *base = k < kLPR ? T : W;
         if (!base) return;
-        const int off = min((k < kLPR ? k : k - kLPR) * 128, kRow - (int)sizeof(float2));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(base + (size_t)y * kRow + off));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(base + G::line(y, k < kLPR ? k : k - kLPR)));
     }
 };
 
@@ -135,7 +135,7 @@ struct L1FirstT {
     const char *T;
     __device__ __forceinline__ void operator()(int y, int k) const {
         if (!T) return;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(T + (size_t)y * kRow + min(k * 128, kRow - (int)sizeof(float2))));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(T + G::line(y, k)));
     }
 };
 
@@ -270,15 +270,25 @@ template <class G, int METHOD, int ADJ, int MODE>
 struct PositionKernel {
     static constexpr int N = G::N, NN = G::N * G::N, R1 = G::R1, R2 = G::R2;
     static constexpr int CB = G::CB;  // points of a column-pass-B task
+    // the saved waves' order: the geometry's (G::grow) in the batched modes,
+    // natural rows where the host reads them back
+    static constexpr bool kLaneW = G::LANES && MODE != kSeq && MODE != kStep;
+    static constexpr int WJ = kLaneW ? G::GJ : R1, WR = kLaneW ? G::GR : N;
+    static __device__ __forceinline__ int wrow(int y) { return kLaneW ? G::grow(y) : y; }
+    static __device__ __forceinline__ size_t wat(int y, int x) {
+        return (size_t)wrow(y) * WR + x % R1 + WJ * (x / R1);
+    }
 
-    // transmission of slab s at (y, x): exp(i sdz sum_{z in slab} V)
+    // transmission of slab s at (y, n1 + R1 j): exp(i sdz sum_{z in slab} V)
     // (mset.cu:134-153 / STEP02_FORWARD_4D.m:12-20; SSET: all z, mset.cu:391-404),
     // read from the precomputed slabs when the tilt has them
-    static __device__ __forceinline__ float2 trans(const LaunchArgs &a, const TiltDev &t, int s, int y, int x) {
+    static __device__ __forceinline__ float2 trans(const LaunchArgs &a, const TiltDev &t, int s, int y, int n1,
+                                                   int j) {
+        const size_t ti = (size_t)s * NN + (size_t)G::grow(y) * G::GR + n1 + G::GJ * j;
         // batched passes always run on precomputed slabs
         if constexpr (MODE == kBatch || MODE == kBatchCk || MODE == kSim)
-            return t.T[(size_t)s * NN + (size_t)y * N + x];
-        if (t.T) return t.T[(size_t)s * NN + (size_t)y * N + x];
+            return t.T[ti];
+        if (t.T) return t.T[ti];
         int z0, z1;
         if constexpr (METHOD == kSSET) {
             z0 = 0;
@@ -287,7 +297,7 @@ struct PositionKernel {
             z0 = s * a.b;
             z1 = min(z0 + a.b, a.nz);
         }
-        const float *p = t.V + (size_t)y * N + x;
+        const float *p = t.V + (size_t)y * N + n1 + R1 * j;
         float acc = 0.f;
         for (int z = z0; z < z1; ++z) acc += p[(size_t)z * NN];
         float sn, cs;
@@ -358,12 +368,12 @@ struct PositionKernel {
             buf, tw,
             [&](int y, int n1, TPre<G> &pre) {
 #pragma unroll
-                for (int j = 0; j < R2; ++j) pre.t[j] = trans(a, t, s0, y, n1 + R1 * j);
+                for (int j = 0; j < R2; ++j) pre.t[j] = trans(a, t, s0, y, n1, j);
             },
             [&](int y, int n1, float2 *v, const TPre<G> &pre) {
-                const float2 *w = ckw + (size_t)y * N + n1;
+                const float2 *w = ckw + (size_t)wrow(y) * WR + n1;
 #pragma unroll
-                for (int j = 0; j < R2; ++j) v[j] = cmul(w[R1 * j], pre.t[j]);
+                for (int j = 0; j < R2; ++j) v[j] = cmul(w[WJ * j], pre.t[j]);
             });
         sync_rows();
         for (int s = s0; s < s1; ++s) {
@@ -377,16 +387,16 @@ struct PositionKernel {
             sync_rows();
             float2 *o = out + (size_t)(s - s0) * NN;
             auto store = [&](int y, int n1, float2 *v) {
-                float2 *w = o + (size_t)y * N + n1;
+                float2 *w = o + (size_t)wrow(y) * WR + n1;
 #pragma unroll
-                for (int j = 0; j < R2; ++j) w[R1 * j] = v[j];
+                for (int j = 0; j < R2; ++j) w[WJ * j] = v[j];
             };
             if (s + 1 < s1) {
                 row_passA_pf<G, +1, -1, TPre<G>>(
                     buf, tw,
                     [&](int y, int n1, TPre<G> &pre) {
 #pragma unroll
-                        for (int j = 0; j < R2; ++j) pre.t[j] = trans(a, t, s + 1, y, n1 + R1 * j);
+                        for (int j = 0; j < R2; ++j) pre.t[j] = trans(a, t, s + 1, y, n1, j);
                     },
                     [&](int y, int n1, float2 *v, const TPre<G> &pre) {
                         store(y, n1, v);
@@ -443,12 +453,12 @@ struct PositionKernel {
         auto pf_t = [&](int s) {
             return [&, s](int y, int n1, TPre<G> &pre) {
                 if constexpr (MODE == kBatch || MODE == kBatchCk || MODE == kSim) {
-                    const float2 *tr = Tslab + (size_t)s * NN + (size_t)y * N + n1;
+                    const float2 *tr = Tslab + (size_t)s * NN + (size_t)G::grow(y) * G::GR + n1;
 #pragma unroll
-                    for (int j = 0; j < R2; ++j) pre.t[j] = tr[R1 * j];
+                    for (int j = 0; j < R2; ++j) pre.t[j] = tr[G::GJ * j];
                 } else {
 #pragma unroll
-                    for (int j = 0; j < R2; ++j) pre.t[j] = trans(a, t, s, y, n1 + R1 * j);
+                    for (int j = 0; j < R2; ++j) pre.t[j] = trans(a, t, s, y, n1, j);
                 }
             };
         };
@@ -469,9 +479,9 @@ struct PositionKernel {
         sync_rows();
         row_passA_pf<G, -1, -1, TPre<G>>(buf, tw, pf_t(0), [&](int y, int n1, float2 *v, const TPre<G> &pre) {
             if constexpr (MODE != kSim && MODE != kErr) {
-                float2 *sv = save + (size_t)y * N + n1;
+                float2 *sv = save + (size_t)wrow(y) * WR + n1;
 #pragma unroll
-                for (int j = 0; j < R2; ++j) sv[R1 * j] = v[j];
+                for (int j = 0; j < R2; ++j) sv[WJ * j] = v[j];
             }
 #pragma unroll
             for (int j = 0; j < R2; ++j) v[j] = cmul(v[j], pre.t[j]);
@@ -514,9 +524,9 @@ struct PositionKernel {
                                 if (w % ck == 0 && w < ns) sv = save + (size_t)(w / ck) * NN;
                             }
                             if (sv) {
-                                sv += (size_t)y * N + n1;
+                                sv += (size_t)wrow(y) * WR + n1;
 #pragma unroll
-                                for (int j = 0; j < R2; ++j) sv[R1 * j] = v[j];
+                                for (int j = 0; j < R2; ++j) sv[WJ * j] = v[j];
                             }
                         }
                         if (!last) {
@@ -670,21 +680,21 @@ struct PositionKernel {
             // loading them inside the op instead (fewer live registers at
             // R2 = 16) exposes their latency and cost 17-22% at n = 256
             auto pf = [&](int y, int n1, APre &pre) {
-                const float2 *sv = wave + (size_t)y * N + n1;
+                const float2 *sv = wave + (size_t)wrow(y) * WR + n1;
                 if constexpr (MODE == kBatch || MODE == kBatchCk) {
                     // the slab row's address once per task (the descriptor
                     // lives in shared memory)
-                    const float2 *tr = Tslab + (size_t)s * NN + (size_t)y * N + n1;
+                    const float2 *tr = Tslab + (size_t)s * NN + (size_t)G::grow(y) * G::GR + n1;
 #pragma unroll
                     for (int j = 0; j < R2; ++j) {
-                        pre.t[j] = tr[R1 * j];
-                        if constexpr (!kStg) pre.w[j] = sv[R1 * j];
+                        pre.t[j] = tr[G::GJ * j];
+                        if constexpr (!kStg) pre.w[j] = sv[WJ * j];
                     }
                 } else {
 #pragma unroll
                     for (int j = 0; j < R2; ++j) {
-                        pre.t[j] = trans(a, t, s, y, n1 + R1 * j);
-                        if constexpr (!kStg) pre.w[j] = sv[R1 * j];
+                        pre.t[j] = trans(a, t, s, y, n1, j);
+                        if constexpr (!kStg) pre.w[j] = sv[WJ * j];
                     }
                 }
                 (void)sv;
@@ -779,14 +789,22 @@ struct PositionKernel {
             for (int i = threadIdx.x; i < G::ROWS * N; i += G::NT) {
                 const int yl = i / N, x = i % N, y = G::gy(yb, yl);
                 const float2 c0 = buf[G::at(yl, x)];
-                const float2 *f = save + (size_t)y * N + x;
                 float2 dx, dy;
-                if (x == 0) dx = csub(f[1], f[0]);
-                else if (x == N - 1) dx = csub(f[0], f[-1]);
-                else dx = cscale(csub(f[1], f[-1]), 0.5f);
-                if (y == 0) dy = csub(f[N], f[0]);
-                else if (y == N - 1) dy = csub(f[0], f[-N]);
-                else dy = cscale(csub(f[N], f[-N]), 0.5f);
+                if constexpr (kLaneW) {
+                    auto f = [&](int yy, int xx) { return save[wat(yy, xx)]; };
+                    dx = csub(f(y, min(x + 1, N - 1)), f(y, max(x - 1, 0)));
+                    dy = csub(f(min(y + 1, N - 1), x), f(max(y - 1, 0), x));
+                    if (x > 0 && x < N - 1) dx = cscale(dx, 0.5f);
+                    if (y > 0 && y < N - 1) dy = cscale(dy, 0.5f);
+                } else {
+                    const float2 *f = save + (size_t)y * N + x;
+                    if (x == 0) dx = csub(f[1], f[0]);
+                    else if (x == N - 1) dx = csub(f[0], f[-1]);
+                    else dx = cscale(csub(f[1], f[-1]), 0.5f);
+                    if (y == 0) dy = csub(f[N], f[0]);
+                    else if (y == N - 1) dy = csub(f[0], f[-N]);
+                    else dy = cscale(csub(f[N], f[-N]), 0.5f);
+                }
                 // Re(conj(d) * chi0)
                 pdx += (double)(dx.x * c0.x + dx.y * c0.y);
                 pdy += (double)(dy.x * c0.x + dy.y * c0.y);
@@ -1111,21 +1129,57 @@ int geo_max_clusters() {
 }
 
 // SEQ: the sequential modes on one CTA (or the batched cluster) per field too,
-// for sessions that turn the split over a cluster off
-template <class G, bool SEQ>
+// for sessions that turn the split over a cluster off; BATCH: the batched modes
+template <class G, bool SEQ, bool BATCH>
 int geo_positions(int method, int adjoint, int mode, const LaunchArgs &a, int grid, cudaStream_t st) {
     if (mode == kErr || mode == kSim) adjoint = kREF;
 #define MSET_L(M, A, MO) \
     if (method == M && adjoint == A && mode == MO) return launch_one<G, M, A, MO>(a, grid, st);
-    MSET_L(kMSET, kREF, kBatch) MSET_L(kMSET, kEXACT, kBatch) MSET_L(kSSET, kREF, kBatch) MSET_L(kSSET, kEXACT, kBatch)
-    MSET_L(kMSET, kREF, kErr) MSET_L(kSSET, kREF, kErr) MSET_L(kMSET, kREF, kSim) MSET_L(kSSET, kREF, kSim)
-    MSET_L(kMSET, kREF, kBatchCk) MSET_L(kMSET, kEXACT, kBatchCk)
+    MSET_L(kMSET, kREF, kErr) MSET_L(kSSET, kREF, kErr)
+    if constexpr (BATCH) {
+        MSET_L(kMSET, kREF, kBatch) MSET_L(kMSET, kEXACT, kBatch) MSET_L(kSSET, kREF, kBatch)
+        MSET_L(kSSET, kEXACT, kBatch) MSET_L(kMSET, kREF, kSim) MSET_L(kSSET, kREF, kSim)
+        MSET_L(kMSET, kREF, kBatchCk) MSET_L(kMSET, kEXACT, kBatchCk)
+    }
     if constexpr (SEQ) {
         MSET_L(kMSET, kREF, kSeq) MSET_L(kMSET, kEXACT, kSeq) MSET_L(kSSET, kREF, kSeq) MSET_L(kSSET, kEXACT, kSeq)
         MSET_L(kMSET, kREF, kStep) MSET_L(kMSET, kEXACT, kStep) MSET_L(kSSET, kREF, kStep) MSET_L(kSSET, kEXACT, kStep)
     }
 #undef MSET_L
     return (int)cudaErrorInvalidValue;
+}
+
+// transmission slabs of every tilt in the geometry's lane order (see
+// k_transmission in mset_dispatch.cu for the natural one)
+template <class G>
+__global__ void k_transmission_lanes(const TiltDev *tilts, int ntilts, int nz, int b, int ns, float sdz) {
+    constexpr int NN = G::N * G::N;
+    const long per = (long)ns * NN, total = per * ntilts;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const long r = i % per;
+        const int s = (int)(r / NN), l = (int)(r % NN);
+        const TiltDev &t = tilts[i / per];
+        int y, x;
+        G::gpos(l, y, x);
+        const int z0 = s * b, z1 = min(z0 + b, nz);
+        float acc = 0.f;
+        for (int z = z0; z < z1; ++z) acc += __ldg(t.V + (size_t)z * NN + y * G::N + x);
+        float sn, cs;
+        sincosf(sdz * acc, &sn, &cs);
+        const_cast<float2 *>(t.T)[r] = make_float2(cs, sn);
+    }
+}
+
+template <class G>
+int geo_transmission(const TiltDev *tilts, int ntilts, int nz, int b, int ns, float sdz, cudaStream_t st) {
+    if constexpr (G::LANES) {
+        const long total = (long)ntilts * ns * G::N * G::N;
+        const int grid = (int)std::min<long>((total + 255) / 256, 148L * 16);
+        k_transmission_lanes<G><<<grid, 256, 0, st>>>(tilts, ntilts, nz, b, ns, sdz);
+        return (int)cudaGetLastError();
+    } else {
+        return launch_transmission(tilts, ntilts, G::N, nz, b, ns, sdz, st);
+    }
 }
 
 template <class G>
@@ -1155,25 +1209,24 @@ int geo_probe_q(bool to_q, const float2 *in, float2 *out, const float2 *twn, cud
 
 }  // namespace mset
 
-// one translation unit per window size defines its table entry; _SEQ: with
-// the sequential modes on this shape
-#define MSET_DEFINE_GEO(N_, R1_, NT_, MINB_) MSET_DEFINE_GEO_T(N_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), false)
-#define MSET_DEFINE_GEO_SEQ(N_, R1_, NT_, MINB_) MSET_DEFINE_GEO_T(N_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), true)
-// another thread / register shape of the same window (same R1, so the same
-// scrambled layouts): a choice for the autotuner, table entry kGeo<NAME_>
-#define MSET_DEFINE_GEO_VARIANT(NAME_, N_, R1_, NT_, MINB_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), false)
+// one translation unit per shape defines its table entry kGeo<NAME_>; _SEQ:
+// with the sequential modes too, _SEQ_ONLY: without the batched ones
+#define MSET_DEFINE_GEO(NAME_, N_, R1_, NT_, MINB_) \
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), false, true)
+#define MSET_DEFINE_GEO_SEQ(NAME_, N_, R1_, NT_, MINB_) \
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), true, true)
+#define MSET_DEFINE_GEO_SEQ_ONLY(NAME_, N_, R1_, NT_, MINB_) \
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (Geo<N_, R1_, NT_, MINB_>), true, false)
 // a field split by rows over a cluster of CL_ CTAs
-#define MSET_DEFINE_GEO_CL(N_, R1_, NT_, CL_) MSET_DEFINE_GEO_T(N_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_>), false)
+#define MSET_DEFINE_GEO_CL(NAME_, N_, R1_, NT_, CL_) \
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_>), false, true)
 // the same with the adjoint's saved-wave rows staged by bulk copies (StageCfg)
 #define MSET_DEFINE_GEO_CL_STAGED(NAME_, N_, R1_, NT_, CL_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, 1, true>), true)
-#define MSET_DEFINE_GEO_CL_VARIANT(NAME_, N_, R1_, NT_, CL_, MINB_) \
-    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, MINB_>), false)
+    MSET_DEFINE_GEO_T(NAME_, N_, R1_, (GeoCl<N_, R1_, NT_, CL_, 1, true>), true, true)
 // the three-phase shape of the 128 x 128 window (Geo3; WIDE_: 16-byte phase-2 accesses)
-#define MSET_DEFINE_GEO3(NAME_, WIDE_) MSET_DEFINE_GEO_T(NAME_, 128, 8, (Geo3<1, WIDE_>), false)
+#define MSET_DEFINE_GEO3(NAME_, WIDE_) MSET_DEFINE_GEO_T(NAME_, 128, 8, (Geo3<1, WIDE_>), false, true)
 #define MSET_UNPAREN(...) __VA_ARGS__
-#define MSET_DEFINE_GEO_T(NAME_, N_, R1_, GT_, SEQ_)                                   \
+#define MSET_DEFINE_GEO_T(NAME_, N_, R1_, GT_, SEQ_, BATCH_)                           \
     namespace mset {                                                                   \
     using Geo##NAME_ = MSET_UNPAREN GT_;                                               \
     extern const GeoOps kGeo##NAME_ = {N_,                                             \
@@ -1184,10 +1237,12 @@ int geo_probe_q(bool to_q, const float2 *in, float2 *out, const float2 *twn, cud
                                        smem_bytes<Geo##NAME_>(),                       \
                                        StageCfg<Geo##NAME_>::kOn ? 1 : 0,              \
                                        SEQ_ ? 1 : 0,                                   \
+                                       BATCH_ ? 1 : 0,                                 \
                                        &geo_max_clusters<Geo##NAME_>,                  \
-                                       &geo_positions<Geo##NAME_, SEQ_>,               \
+                                       &geo_positions<Geo##NAME_, SEQ_, BATCH_>,       \
                                        &geo_prep_amp<Geo##NAME_>,                      \
                                        &geo_prep_amp_bf16<Geo##NAME_>,                 \
                                        &geo_prep_prop<Geo##NAME_>,                     \
-                                       &geo_probe_q<Geo##NAME_>};                      \
+                                       &geo_probe_q<Geo##NAME_>,                       \
+                                       &geo_transmission<Geo##NAME_>};                 \
     }
