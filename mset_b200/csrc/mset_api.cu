@@ -156,7 +156,7 @@ struct mset_session {
     cudaGraphExec_t phase_exec[2] = {nullptr, nullptr};
     int grid_cache = 0;
     // TV work buffers
-    DevBuf<float> tv_in, tv_out, tv_P, tv_Y, tv_D;
+    DevBuf<float> tv_in, tv_out, tv_P, tv_Y, tv_Y2, tv_D;
     DevBuf<double> tv_err;
     // rotation work buffers
     // per-position steps (mset_forward_position / mset_adjoint_position)
@@ -1281,6 +1281,16 @@ int mset_rotate_volume(mset_session *s, const float *vol_in, float *vol_out, int
 }
 
 // ---- TV / TV-FISTA ----------------------------------------------------------
+// the second momentum field where it saves a kernel per iteration; without the
+// memory for it TV runs on what it has
+static int tv_second(mset_session *s, int n1, int n2, int n3, int fista) {
+    const size_t want = tv_wants_second(n1, n2, n3, fista != 0) ? 3 * (size_t)n1 * n2 * n3 : 0;
+    const cudaError_t e = s->tv_Y2.n < want ? s->tv_Y2.ensure(want) : cudaSuccess;
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    else if (e != cudaSuccess) return cuda_fail(e, "allocating the TV work field");
+    return 0;
+}
+
 int mset_tv(mset_session *s, float *vol, int n1, int n2, int n3, double lambda, int niter, int fista,
             double *tv_error) {
     Range range_("mset_tv");
@@ -1296,10 +1306,12 @@ int mset_tv(mset_session *s, float *vol, int n1, int n2, int n3, double lambda, 
     CK(s->tv_Y.ensure(3 * V));
     CK(s->tv_D.ensure(V));
     CK(s->tv_err.ensure(1));
+    rc = tv_second(s, n1, n2, n3, fista);
+    if (rc) return rc;
     CK(cudaMemcpyAsync(s->tv_in.p, vol, sizeof(float) * V, cudaMemcpyHostToDevice, s->st));
     CK(cudaMemsetAsync(s->tv_err.p, 0, sizeof(double), s->st));
     TvArgs a{s->tv_in.p, s->tv_out.p, s->tv_P.p, s->tv_Y.p, s->tv_D.p, n1, n2, n3, lambda, niter, fista ? 1 : 0,
-             s->tv_err.p};
+             s->tv_err.p, s->tv_Y2.p};
     CKL(tv_prox(a, s->st), "tv");
     CK(cudaMemcpyAsync(vol, s->tv_out.p, sizeof(float) * V, cudaMemcpyDeviceToHost, s->st));
     double e = 0;
@@ -1386,6 +1398,8 @@ int mset_batch_iteration_setup_nd(mset_session *s, const mset_iter_args *a, int 
         CK(s->tv_Y.ensure(3 * V));
         CK(s->tv_D.ensure(V));
         CK(s->tv_err.ensure(1));
+        rc = tv_second(s, nv1, nv2, nv3, s->it_tv_fista);
+        if (rc) return rc;
     }
     CK(cudaStreamSynchronize(s->st));
     drop_graph(s);
@@ -1466,7 +1480,7 @@ update:
         CKL(vol_scale(s->rec.p, s->tv_in.p, V, s->mx.p, s->st), "scale");
         CK(cudaMemsetAsync(s->tv_err.p, 0, sizeof(double), s->st));
         const TvArgs ta{s->tv_in.p, s->tv_out.p, s->tv_P.p, s->tv_Y.p, s->tv_D.p, s->nv1, s->nv2, s->nv3,
-                        s->it_tv_lambda, s->it_tv_iter, s->it_tv_fista, s->tv_err.p};
+                        s->it_tv_lambda, s->it_tv_iter, s->it_tv_fista, s->tv_err.p, s->tv_Y2.p};
         CKL(tv_prox(ta, s->st), "tv");
         CKL(vol_mul(s->tv_out.p, s->rec.p, V, s->mx.p, s->st), "rescale");
     }
@@ -1542,7 +1556,7 @@ static int record_tv(mset_session *s) {
     CKL(vol_scale(s->rec.p, s->tv_in.p, V, s->mx.p, s->st), "scale");
     CK(cudaMemsetAsync(s->tv_err.p, 0, sizeof(double), s->st));
     const TvArgs ta{s->tv_in.p, s->tv_out.p, s->tv_P.p, s->tv_Y.p, s->tv_D.p, s->nv1, s->nv2, s->nv3,
-                    s->it_tv_lambda, s->it_tv_iter, s->it_tv_fista, s->tv_err.p};
+                    s->it_tv_lambda, s->it_tv_iter, s->it_tv_fista, s->tv_err.p, s->tv_Y2.p};
     CKL(tv_prox(ta, s->st), "tv");
     CKL(vol_mul(s->tv_out.p, s->rec.p, V, s->mx.p, s->st), "rescale");
     return 0;

@@ -7,10 +7,14 @@
 // All stencils are periodic (MATLAB circshift).  Volumes are C order
 // [n3][n2][n1] = MATLAB (n1, n2, n3); MATLAB dim 1 is the fastest axis.
 // HBM/L2-bound elementwise work: grid-stride loops over 148 x 8 CTAs (the
-// TV stencils: over rows, one CTA per row).
+// scalar TV stencils: over rows, one CTA per row).  TV runs on one of three
+// routes (tv_prox): every iteration in one cluster launch where the volume fits
+// its shared memory, one marching kernel per iteration where rows are whole
+// float4 groups, else two kernels per iteration.
 #include <algorithm>
 #include <cmath>
 
+#include "fft_core.cuh"
 #include "mset_volume.cuh"
 
 namespace mset {
@@ -120,36 +124,13 @@ __global__ void k_tv_err(const float *u, Rows g, double lam, double *err) {
     if ((threadIdx.x & 31) == 0) atomicAdd(err, lam * acc);
 }
 
-// The same three stencils with four consecutive voxels per thread (n1 a
-// multiple of 4): 16-byte loads and stores of every array, the one periodic
-// neighbour along i1 outside the thread's four voxels read as a 4-byte load
-// (an L1 hit: the neighbouring thread loads its line).  Fewer, wider requests
-// keep more bytes in flight per SM; same arithmetic per voxel.
+// Four consecutive voxels per thread (n1 a multiple of 4): 16-byte loads and
+// stores of every array, the one periodic neighbour along i1 outside the
+// thread's four voxels read as a 4-byte load (an L1 hit: the neighbouring
+// thread loads its line).  Fewer, wider requests keep more bytes in flight per
+// SM; same arithmetic per voxel.
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
-
-__global__ void k_tv_d4(const float *Y, const float *in, float *D, Rows g, float inv_lam) {
-    const long V = g.V;
-    const int q1 = g.n1 / 4;
-    for (int row = blockIdx.x; row < g.n2 * g.n3; row += gridDim.x) {
-        const int i2 = row % g.n2, i3 = row / g.n2;
-        const long b = g.at(i2, i3), b2 = g.at(i2 == 0 ? g.n2 - 1 : i2 - 1, i3),
-                   b3 = g.at(i2, i3 == 0 ? g.n3 - 1 : i3 - 1);
-        for (int k = threadIdx.x; k < q1; k += blockDim.x) {
-            const int i1 = 4 * k;
-            const long r = b + i1;
-            const float4 y1 = ld4(Y + r), y2 = ld4(Y + V + r), y3 = ld4(Y + 2 * V + r);
-            const float4 m2 = ld4(Y + V + b2 + i1), m3 = ld4(Y + 2 * V + b3 + i1), u = ld4(in + r);
-            const float y1m = Y[b + (i1 == 0 ? g.n1 - 1 : i1 - 1)];
-            float4 d;
-            d.x = (y1.x + y2.x + y3.x - y1m - m2.x - m3.x) - u.x * inv_lam;
-            d.y = (y1.y + y2.y + y3.y - y1.x - m2.y - m3.y) - u.y * inv_lam;
-            d.z = (y1.z + y2.z + y3.z - y1.y - m2.z - m3.z) - u.z * inv_lam;
-            d.w = (y1.w + y2.w + y3.w - y1.z - m2.w - m3.w) - u.w * inv_lam;
-            st4(D + r, d);
-        }
-    }
-}
 
 __device__ __forceinline__ void tv_project(float q1, float q2, float q3, float &p1, float &p2, float &p3) {
     const float nrm = sqrtf(fmaxf(1.0f, q1 * q1 + q2 * q2 + q3 * q3));
@@ -158,52 +139,225 @@ __device__ __forceinline__ void tv_project(float q1, float q2, float q3, float &
     p3 = q3 / nrm;
 }
 
-__global__ void k_tv_step4(float *P, float *Y, const float *D, Rows g, float tau, double m, int fista) {
+// One iteration as one kernel (rows of whole float4 groups): D = div(src) -
+// in / lambda is never stored.  A CTA takes ty adjacent rows of a slice, full
+// length, and marches through zc slices: per slice it computes D of the next
+// one (its rows and the row above them) from that slice's dual values, which
+// stay in registers as the next step's source, leaves it in shared memory for
+// the neighbours along i1 and i2, and finishes the current slice.  The dual
+// field is read from src and written to dst, so the neighbours' old values
+// survive.  Per voxel it moves 16 B of source and input (and 1 / zc + 1 / ty
+// of them again), 12 of P and 24 of results, against 20 + 52 in two kernels
+// with D in memory, and half the launches: 164.8 -> 113.4 us per FISTA iteration
+// at 256 x 256 x 192 (6.0 TB/s of HBM), 24.8 -> 20.6 at 128^3 (L2 and the
+// chain of a step), 16.3 -> 10.3 at 96^3.
+struct Quad {
+    float v[4];
+};
+__device__ __forceinline__ Quad quad(const float *p) {
+    const float4 q = ld4(p);
+    return Quad{{q.x, q.y, q.z, q.w}};
+}
+__device__ __forceinline__ void put(float *p, const Quad &q) { st4(p, make_float4(q.v[0], q.v[1], q.v[2], q.v[3])); }
+
+// D of four voxels at row offset b (+ i1) with the neighbours' rows b2 (i2 - 1)
+// and m3 = Y3 one slice below; the dual values come back in y
+__device__ __forceinline__ Quad tv_d4(const float *Y, const float *in, long V, long b, long b2, int i1, int n1,
+                                      float inv_lam, const Quad &m3, Quad y[3]) {
+    const Quad m2 = quad(Y + V + b2 + i1), u = quad(in + b + i1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[c] = quad(Y + c * V + b + i1);
+    const float y1m = Y[b + (i1 == 0 ? n1 - 1 : i1 - 1)];
+    Quad d;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        d.v[e] = (y[0].v[e] + y[1].v[e] + y[2].v[e] - (e ? y[0].v[e ? e - 1 : 0] : y1m) - m2.v[e] - m3.v[e]) -
+                 u.v[e] * inv_lam;
+    return d;
+}
+
+template <bool FISTA>
+__global__ void __launch_bounds__(256) k_tv_march(const float *src, float *dst, float *P, const float *in, Rows g,
+                                                  int ty, int zc, float inv_lam, float tau, double m) {
+    extern __shared__ __align__(16) float dsm[];
     const long V = g.V;
-    const int q1 = g.n1 / 4;
-    for (int row = blockIdx.x; row < g.n2 * g.n3; row += gridDim.x) {
-        const int i2 = row % g.n2, i3 = row / g.n2;
-        const long b = g.at(i2, i3), b2 = g.at(i2 == g.n2 - 1 ? 0 : i2 + 1, i3),
-                   b3 = g.at(i2, i3 == g.n3 - 1 ? 0 : i3 + 1);
-        for (int k = threadIdx.x; k < q1; k += blockDim.x) {
-            const int i1 = 4 * k;
-            const long r = b + i1;
-            const float4 d0 = ld4(D + r), dn2 = ld4(D + b2 + i1), dn3 = ld4(D + b3 + i1);
-            const float dp = D[b + (i1 + 4 == g.n1 ? 0 : i1 + 4)];
-            const float *src = fista ? Y : P;
-            const float4 s1 = ld4(src + r), s2 = ld4(src + V + r), s3 = ld4(src + 2 * V + r);
-            const float d[5] = {d0.x, d0.y, d0.z, d0.w, dp};
-            const float e2[4] = {dn2.x, dn2.y, dn2.z, dn2.w}, e3[4] = {dn3.x, dn3.y, dn3.z, dn3.w};
-            const float a1[4] = {s1.x, s1.y, s1.z, s1.w}, a2[4] = {s2.x, s2.y, s2.z, s2.w},
-                        a3[4] = {s3.x, s3.y, s3.z, s3.w};
-            float o1[4], o2[4], o3[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float t1 = tau * (d[e + 1] - d[e]);
-                const float t2 = tau * (e2[e] - d[e]);
-                const float t3 = tau * (e3[e] - d[e]);
-                tv_project(a1[e] + t1, a2[e] + t2, a3[e] + t3, o1[e], o2[e], o3[e]);
-            }
-            if (fista) {
-                const float4 p1 = ld4(P + r), p2 = ld4(P + V + r), p3 = ld4(P + 2 * V + r);
-                const float b1[4] = {p1.x, p1.y, p1.z, p1.w}, b2v[4] = {p2.x, p2.y, p2.z, p2.w},
-                            b3v[4] = {p3.x, p3.y, p3.z, p3.w};
-                float y1[4], y2[4], y3[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    y1[e] = (float)(o1[e] + m * (o1[e] - (double)b1[e]));
-                    y2[e] = (float)(o2[e] + m * (o2[e] - (double)b2v[e]));
-                    y3[e] = (float)(o3[e] + m * (o3[e] - (double)b3v[e]));
-                }
-                st4(Y + r, make_float4(y1[0], y1[1], y1[2], y1[3]));
-                st4(Y + V + r, make_float4(y2[0], y2[1], y2[2], y2[3]));
-                st4(Y + 2 * V + r, make_float4(y3[0], y3[1], y3[2], y3[3]));
-            }
-            st4(P + r, make_float4(o1[0], o1[1], o1[2], o1[3]));
-            st4(P + V + r, make_float4(o2[0], o2[1], o2[2], o2[3]));
-            st4(P + 2 * V + r, make_float4(o3[0], o3[1], o3[2], o3[3]));
+    const int q1 = g.n1 / 4, i1 = 4 * (threadIdx.x % q1), r = threadIdx.x / q1;
+    const int tiles = (g.n2 + ty - 1) / ty;
+    const int y0 = (blockIdx.x % tiles) * ty, z0 = (blockIdx.x / tiles) * zc, z1 = min(z0 + zc, g.n3);
+    const int rows = min(ty, g.n2 - y0);
+    const bool on = r < rows, halo = r == 0;
+    const int y = y0 + (on ? r : 0), ym = y == 0 ? g.n2 - 1 : y - 1;
+    const int yh = y0 + rows == g.n2 ? 0 : y0 + rows, yhm = y0 + rows - 1;
+    float *cur = dsm, *nxt = dsm + (ty + 1) * g.n1;
+    Quad yc[3], d0;
+    {
+        const int zm = z0 == 0 ? g.n3 - 1 : z0 - 1;
+        if (on) {
+            d0 = tv_d4(src, in, V, g.at(y, z0), g.at(ym, z0), i1, g.n1, inv_lam, quad(src + 2 * V + g.at(y, zm) + i1), yc);
+            put(cur + r * g.n1 + i1, d0);
+        }
+        if (halo) {
+            Quad yy[3];
+            put(cur + rows * g.n1 + i1, tv_d4(src, in, V, g.at(yh, z0), g.at(yhm, z0), i1, g.n1, inv_lam,
+                                              quad(src + 2 * V + g.at(yh, zm) + i1), yy));
         }
     }
+    __syncthreads();
+    for (int z = z0; z < z1; ++z) {
+        const int zp = z + 1 == g.n3 ? 0 : z + 1;
+        Quad yn[3], dn, p[3];
+        if (on) {
+            const long o = g.at(y, z) + i1;
+            if constexpr (FISTA) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) p[c] = quad(P + c * V + o);
+            }
+            dn = tv_d4(src, in, V, g.at(y, zp), g.at(ym, zp), i1, g.n1, inv_lam, yc[2], yn);
+            put(nxt + r * g.n1 + i1, dn);
+            const float *row = cur + r * g.n1;
+            const float dp = row[i1 + 4 == g.n1 ? 0 : i1 + 4];
+            const Quad du = quad(row + g.n1 + i1);
+            Quad w[3];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float t1 = tau * ((e < 3 ? d0.v[e < 3 ? e + 1 : 3] : dp) - d0.v[e]);
+                const float t2 = tau * (du.v[e] - d0.v[e]);
+                const float t3 = tau * (dn.v[e] - d0.v[e]);
+                tv_project(yc[0].v[e] + t1, yc[1].v[e] + t2, yc[2].v[e] + t3, w[0].v[e], w[1].v[e], w[2].v[e]);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if constexpr (FISTA) {
+                    Quad f;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) f.v[e] = (float)(w[c].v[e] + m * (w[c].v[e] - (double)p[c].v[e]));
+                    put(dst + c * V + o, f);
+                    put(P + c * V + o, w[c]);
+                } else {
+                    put(dst + c * V + o, w[c]);
+                }
+                yc[c] = yn[c];
+            }
+            d0 = dn;
+        }
+        if (halo && z + 1 < z1) {
+            Quad yy[3];
+            put(nxt + rows * g.n1 + i1, tv_d4(src, in, V, g.at(yh, zp), g.at(yhm, zp), i1, g.n1, inv_lam,
+                                              quad(src + 2 * V + g.at(yh, z) + i1), yy));
+        }
+        __syncthreads();
+        float *s = cur;
+        cur = nxt;
+        nxt = s;
+    }
+}
+
+// All iterations of a small volume in one launch: the slices are dealt out over
+// a cluster, K per CTA, and the dual fields stay in shared memory.  Launches
+// bound the kernels above at these sizes; here it is the arithmetic of one
+// CTA's slices (square root, three divisions, FP64 momentum per voxel), so the
+// cluster is the largest one (24^3: 8.1 us per iteration of two launches, 2.5 on
+// 8 CTAs, 1.9 on 16; 32^3: 8.2, 6.6, 4.1).  Per iteration a CTA
+// computes D of its slices and of the one above them, steps, and hands its
+// bottom slice's new dual values to the CTA below and its top slice's third
+// component to the CTA above (two halo buffers in turn, so one cluster barrier
+// per iteration orders both the reads and the writes).  A thread of a warp of
+// its own works out the next momentum factor meanwhile.
+constexpr int kTvCl = 16;  // 8 where the device holds no cluster of 16
+
+// floats of shared memory for planes of `plane` voxels, K slices per CTA
+inline long tv_cluster_floats(long plane, int K, bool fista) {
+    return plane * ((fista ? 6L : 3L) * K + 2L * (K + 1) + 8);
+}
+
+template <bool FISTA>
+__global__ void __launch_bounds__(1024) k_tv_cluster(float *Pout, const float *in, Rows g, int K, float inv_lam,
+                                                     float tau, int niter) {
+    extern __shared__ __align__(16) float dsm[];
+    __shared__ double s_m[2];
+    const int A = g.n1 * g.n2, lanes = blockDim.x - 32, tid = threadIdx.x;
+    unsigned rk;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rk));
+    const int rank = (int)rk, z0 = rank * K, busy = (g.n3 + K - 1) / K;
+    const int own = max(0, min(K, g.n3 - z0));
+    float *Y = dsm, *Pp = Y + 3 * K * A, *U = Pp + (FISTA ? 3 * K * A : 0), *D = U + (K + 1) * A;
+    float *hy = D + (K + 1) * A, *hz = hy + 6 * A;  // [2][3][A] and [2][A]
+    for (int i = tid; i < (FISTA ? 6 : 3) * K * A; i += blockDim.x) Y[i] = 0.f;
+    for (int i = tid; i < 8 * A; i += blockDim.x) hy[i] = 0.f;
+    if (own)
+        for (int i = tid; i < (own + 1) * A; i += blockDim.x) U[i] = in[(long)((z0 + i / A) % g.n3) * A + i % A];
+    float *const below = peer(hy, (rank + busy - 1) % busy), *const above = peer(hz, (rank + 1) % busy);
+    // this thread's first column and its neighbours; others are found as met
+    int xm, ym, xp, yp;
+    auto column = [&](int c) {
+        const int i1 = c % g.n1;
+        xm = i1 == 0 ? c + g.n1 - 1 : c - 1;
+        ym = c < g.n1 ? c + A - g.n1 : c - g.n1;
+        xp = i1 + 1 == g.n1 ? c - i1 : c + 1;
+        yp = c + g.n1 < A ? c + g.n1 : i1;
+    };
+    const bool work = own && tid < lanes, one = A <= lanes;
+    column(tid);
+    double t = 1.0;
+    auto momentum = [&](int h) {  // TV_FISTA_method.m:31, rounded as on the host
+        const double t0 = t;
+        t = __ddiv_rn(__dadd_rn(1.0, __dsqrt_rn(__dadd_rn(1.0, __dmul_rn(__dmul_rn(4.0, t0), t0)))), 2.0);
+        s_m[h] = __ddiv_rn(t0 - 1.0, t);
+    };
+    const bool clock = FISTA && tid == (int)blockDim.x - 1;
+    if (clock) momentum(0);
+    cluster_sync();
+    for (int it = 0; it < niter; ++it) {
+        const int h = it & 1;
+        const float *hyc = hy + 3 * h * A, *hzc = hz + h * A;
+        if (work)
+            for (int c = tid; c < A; c += lanes) {
+                if (!one) column(c);
+                float y3m = hzc[c];
+                for (int k = 0; k <= own; ++k) {
+                    const float *q = k < own ? Y + 3 * k * A : hyc;
+                    const float y3 = q[2 * A + c];
+                    const float d = q[c] + q[A + c] + y3 - q[xm] - q[A + ym] - y3m;
+                    D[k * A + c] = d - U[k * A + c] * inv_lam;
+                    y3m = y3;
+                }
+            }
+        __syncthreads();
+        if (work) {
+            const double m = FISTA ? s_m[h] : 0.0;
+            for (int c = tid; c < A; c += lanes) {
+                if (!one) column(c);
+                for (int k = 0; k < own; ++k) {
+                    const float *dk = D + k * A;
+                    float *q = Y + 3 * k * A + c;
+                    const float d0 = dk[c];
+                    const float t1 = tau * (dk[xp] - d0);
+                    const float t2 = tau * (dk[yp] - d0);
+                    const float t3 = tau * (dk[A + c] - d0);
+                    float p[3], f[3];
+                    tv_project(q[0] + t1, q[A] + t2, q[2 * A] + t3, p[0], p[1], p[2]);
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) {
+                        f[e] = p[e];
+                        if constexpr (FISTA) {
+                            float *o = Pp + (3 * k + e) * A + c;
+                            f[e] = (float)(p[e] + m * (p[e] - (double)*o));
+                            *o = p[e];
+                        }
+                        q[e * A] = f[e];
+                        if (k == 0) below[(3 * (h ^ 1) + e) * A + c] = f[e];
+                    }
+                    if (k == own - 1) above[(h ^ 1) * A + c] = f[2];
+                }
+            }
+        } else if (clock) {
+            momentum(h ^ 1);
+        }
+        cluster_sync();
+    }
+    const float *res = FISTA ? Pp : Y;
+    for (int i = tid; i < 3 * own * A; i += blockDim.x)
+        Pout[(i / A % 3) * g.V + (long)(z0 + i / (3 * A)) * A + i % A] = res[i];
 }
 
 __global__ void k_tv_out4(const float *P, const float *in, float *out, Rows g, float lam) {
@@ -303,6 +457,54 @@ __global__ void k_update(float *rec, const double *acc, long n, float step0) {
 }
 }  // namespace
 
+namespace {
+// launch configuration of the cluster kernel over a volume; false: it does not
+// fit one cluster's shared memory
+template <bool FISTA>
+struct TvCluster {
+    cudaLaunchAttribute at[1] = {};
+    cudaLaunchConfig_t cfg = {};
+    int K = 0;
+    bool prepare(int n1, int n2, int n3, cudaStream_t st) {
+        const long A = (long)n1 * n2;
+        for (int cl : {kTvCl, 8}) {
+            K = (n3 + cl - 1) / cl;
+            const long bytes = tv_cluster_floats(A, K, FISTA) * (long)sizeof(float);
+            if (bytes > 220 * 1024) continue;
+            auto k = k_tv_cluster<FISTA>;
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+                (cl > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
+                return false;
+            cfg.gridDim = dim3(cl);
+            cfg.blockDim = dim3((unsigned)std::min(992L, (A + 31) / 32 * 32) + 32);
+            cfg.dynamicSmemBytes = (size_t)bytes;
+            cfg.stream = st;
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = cl;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cl <= 8 || (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0)) return true;
+        }
+        return false;
+    }
+};
+// every iteration in one launch; -1: the volume does not fit
+template <bool FISTA>
+int tv_cluster(const TvArgs &a, const Rows &rows, float inv_lam, float tau, cudaStream_t st) {
+    TvCluster<FISTA> c;
+    if (!c.prepare(a.n1, a.n2, a.n3, st)) return -1;
+    return (int)cudaLaunchKernelEx(&c.cfg, k_tv_cluster<FISTA>, a.P, a.in, rows, c.K, inv_lam, tau, a.niter);
+}
+}  // namespace
+
+bool tv_wants_second(int n1, int n2, int n3, bool fista) {
+    TvCluster<true> c;
+    return fista && n1 % 4 == 0 && n1 <= 1024 && !c.prepare(n1, n2, n3, nullptr);
+}
+
 int tv_prox(const TvArgs &a, cudaStream_t st) {
     const long V = (long)a.n1 * a.n2 * a.n3;
     const Rows rows{a.n1, a.n2, a.n3, V};
@@ -313,27 +515,58 @@ int tv_prox(const TvArgs &a, cudaStream_t st) {
     // four voxels per thread where rows split into 16-byte groups (every
     // array is 16-byte aligned and n1 a multiple of 4)
     const bool vec = a.n1 % 4 == 0;
-    const int bt4 = std::min(256, (a.n1 / 4 + 31) / 32 * 32);
+    const int bt4 = std::min(256, std::max(1, (a.n1 / 4 + 31) / 32) * 32);
     const int g4 = (int)std::min<long>((long)a.n2 * a.n3, 148L * std::min(32, 2048 / bt4));
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(a.P, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemsetAsync(a.Y, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
     const float tau = 1.0f / 12.0f;  // 3D (TV_method.m:13-16)
-    double t = 1.0;
-    for (int it = 0; it < a.niter; ++it) {
-        const double t0 = t;
-        t = (1.0 + std::sqrt(1.0 + 4.0 * t0 * t0)) / 2.0;  // TV_FISTA_method.m:31
-        const double m = (t0 - 1.0) / t;
-        if (vec) {
-            k_tv_d4<<<g4, bt4, 0, st>>>(a.fista ? a.Y : a.P, a.in, a.D, rows, (float)(1.0 / a.lambda));
-            k_tv_step4<<<g4, bt4, 0, st>>>(a.P, a.Y, a.D, rows, tau, m, a.fista);
-        } else {
-            k_tv_d<<<g, bt, 0, st>>>(a.fista ? a.Y : a.P, a.in, a.D, rows, (float)(1.0 / a.lambda));
-            k_tv_step<<<g, bt, 0, st>>>(a.P, a.Y, a.D, rows, tau, m, a.fista);
+    const float inv_lam = (float)(1.0 / a.lambda);
+    float *res = a.P;  // the dual field after the last iteration
+    cudaError_t e;
+    int rc = -1;
+    if (a.niter > 0) rc = a.fista ? tv_cluster<true>(a, rows, inv_lam, tau, st) : tv_cluster<false>(a, rows, inv_lam, tau, st);
+    if (rc > 0) return rc;
+    if (rc < 0) {
+        if ((e = cudaMemsetAsync(a.P, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
+        if ((e = cudaMemsetAsync(a.Y, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
+        // one kernel per iteration needs a second dual field: Y2 (FISTA), or P
+        // and Y in turn
+        const bool march = vec && a.n1 <= 1024 && (!a.fista || a.Y2);
+        const int q1 = std::max(1, a.n1 / 4), ty = std::max(1, std::min(128 / q1, a.n2));
+        const int tiles = (a.n2 + ty - 1) / ty;
+        int zc = 1;
+        double best = 0;
+        for (int c = 1; c <= std::min(16, a.n3); ++c) {
+            // chunks of c slices (0.6 more for a chunk's start) in waves of the
+            // 6 CTAs an SM holds; a wave less than two thirds full takes as
+            // long as one, half of a last wave's empty places are lost (128^3:
+            // 17.6 us at c = 5, 0.94 waves; 21.2 at 4, 1.15; 18.0 at 3; 24.0 at 1)
+            const double w = (double)tiles * ((a.n3 + c - 1) / c) / (148.0 * 6.0), up = std::ceil(w);
+            const double cost = (c + 0.6) * (w <= 1.0 ? std::max(w, 0.65) : 0.5 * (w + up));
+            if (c == 1 || cost < best) {
+                best = cost;
+                zc = c;
+            }
         }
+        const int grid = tiles * ((a.n3 + zc - 1) / zc);
+        const size_t sm = sizeof(float) * 2 * (size_t)(ty + 1) * a.n1;
+        float *src = a.fista ? a.Y : a.P, *dst = a.fista ? a.Y2 : a.Y;
+        double t = 1.0;
+        for (int it = 0; it < a.niter; ++it) {
+            const double t0 = t;
+            t = (1.0 + std::sqrt(1.0 + 4.0 * t0 * t0)) / 2.0;  // TV_FISTA_method.m:31
+            const double m = (t0 - 1.0) / t;
+            if (march) {
+                if (a.fista) k_tv_march<true><<<grid, q1 * ty, sm, st>>>(src, dst, a.P, a.in, rows, ty, zc, inv_lam, tau, m);
+                else k_tv_march<false><<<grid, q1 * ty, sm, st>>>(src, dst, nullptr, a.in, rows, ty, zc, inv_lam, tau, m);
+                std::swap(src, dst);
+            } else {
+                k_tv_d<<<g, bt, 0, st>>>(a.fista ? a.Y : a.P, a.in, a.D, rows, inv_lam);
+                k_tv_step<<<g, bt, 0, st>>>(a.P, a.Y, a.D, rows, tau, m, a.fista);
+            }
+        }
+        if (march && !a.fista) res = src;
     }
-    if (vec) k_tv_out4<<<g4, bt4, 0, st>>>(a.P, a.in, a.out, rows, (float)a.lambda);
-    else k_tv_out<<<g, bt, 0, st>>>(a.P, a.in, a.out, rows, (float)a.lambda);
+    if (vec) k_tv_out4<<<g4, bt4, 0, st>>>(res, a.in, a.out, rows, (float)a.lambda);
+    else k_tv_out<<<g, bt, 0, st>>>(res, a.in, a.out, rows, (float)a.lambda);
     if (a.err) k_tv_err<<<g, bt, 0, st>>>(a.out, rows, a.lambda, a.err);
     return (int)cudaGetLastError();
 }

@@ -14,7 +14,12 @@ struct TvArgs {
     int niter;
     int fista;               // 1: TV_FISTA_method, 0: TV_method
     double *err;             // optional device accumulator: += lambda * TV_error(output)
+    float *Y2;               // [3][V] second momentum field (tv_wants_second), or null: two
+                             // kernels per iteration
 };
+
+// whether an iteration runs as one kernel given a second momentum field
+bool tv_wants_second(int n1, int n2, int n3, bool fista);
 
 int tv_prox(const TvArgs &a, cudaStream_t st);
 int vol_max(const float *v, long n, unsigned *bits, float *mx, cudaStream_t st);
