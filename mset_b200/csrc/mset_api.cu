@@ -167,6 +167,7 @@ struct mset_session {
     float step_x = 0, step_y = 0;
     DevBuf<float> rot_vol;
     DevBuf<float2> rot_S, rot_tw;
+    int rot_group = 1;  // cubic reconstruction: tilts rotated at once
     int rot_n = 0;
 };
 
@@ -1228,10 +1229,74 @@ static int rot_prepare(mset_session *s, int n) {
     return 0;
 }
 
-// rotation of the reconstruction-shaped volume src into dst (may alias)
-static int rotate_rec(mset_session *s, const RotPlan &pl, const float *src, float *dst) {
-    if (s->nv > 0) return rot_apply(pl, s->nv, src, dst, s->rot_S.p, s->rot_tw.p, s->sms, s->st);
-    return rot_apply3(pl, s->nv1, s->nv2, s->nv3, src, dst, s->rot_S.p, s->sms, s->st);
+// work volumes for rotating several tilts of a cubic reconstruction at once,
+// up to 64 MB of them (one is there already; without memory for more, one)
+static int rot_prepare_group(mset_session *s, int n, int tilts) {
+    const size_t nvox = (size_t)n * n * n;
+    const size_t fit = std::max<size_t>(1, ((size_t)64 << 20) / (sizeof(float2) * nvox));
+    s->rot_group = (int)std::min<size_t>({fit, (size_t)kRotJobs, (size_t)std::max(1, tilts)});
+    if (s->rot_S.n >= s->rot_group * nvox) return 0;
+    cudaError_t e = s->rot_S.ensure(s->rot_group * nvox);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        s->rot_group = 1;
+        e = s->rot_S.ensure(nvox);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "allocating rotation work volumes");
+    return 0;
+}
+
+// V_j = pad(Func_inv_rot(rec, angles_j)) of every tilt (STEP01_ROTATION.m:13)
+static int rec_to_tilts(mset_session *s) {
+    const int J = (int)s->tilts.size();
+    if (s->nv == 0) {
+        for (int j = 0; j < J; ++j) {
+            CKL(rot_apply3(s->plan_inv[j], s->nv1, s->nv2, s->nv3, s->rec.p, s->gvol.p, s->rot_S.p, s->sms, s->st),
+                "rotation");
+            CKL(vol_pad(s->gvol.p, s->tilts[j].V.p, s->nv1, s->nv2, s->nv3, s->n, s->st), "pad");
+        }
+        return 0;
+    }
+    for (int j0 = 0; j0 < J; j0 += s->rot_group) {
+        const int count = std::min(s->rot_group, J - j0);
+        const RotPlan *pl[kRotJobs];
+        float *V[kRotJobs];
+        for (int j = 0; j < count; ++j) {
+            pl[j] = &s->plan_inv[j0 + j];
+            V[j] = s->tilts[j0 + j].V.p;
+        }
+        CKL(rot_to_windows(pl, count, s->nv, s->rec.p, V, s->n, s->rot_S.p, s->rot_tw.p, s->sms, s->st), "rotation");
+    }
+    return 0;
+}
+
+// gacc = sum_j Func_rot(G_j) (Run_MSET_recon.m:179)
+static int tilts_to_gacc(mset_session *s, int bvox) {
+    const int J = (int)s->tilts.size();
+    if (s->nv == 0) {
+        const long V = (long)s->nv1 * s->nv2 * s->nv3;
+        for (int j = 0; j < J; ++j) {
+            CKL(vol_slab_to_volume(s->tilts[j].grad.p, s->gvol.p, s->nv1, s->nv2, s->nv3, s->n, bvox, s->st),
+                "slab_to_volume");
+            CKL(rot_apply3(s->plan_fwd[j], s->nv1, s->nv2, s->nv3, s->gvol.p, s->gvol.p, s->rot_S.p, s->sms, s->st),
+                "rotation");
+            CKL(vol_accumulate(s->gvol.p, s->gacc.p, V, j == 0, s->st), "accumulate");
+        }
+        return 0;
+    }
+    for (int j0 = 0; j0 < J; j0 += s->rot_group) {
+        const int count = std::min(s->rot_group, J - j0);
+        const RotPlan *pl[kRotJobs];
+        const double *G[kRotJobs];
+        for (int j = 0; j < count; ++j) {
+            pl[j] = &s->plan_fwd[j0 + j];
+            G[j] = s->tilts[j0 + j].grad.p;
+        }
+        CKL(rot_accumulate(pl, count, s->nv, G, s->n, bvox, s->gacc.p, j0 == 0, s->rot_S.p, s->rot_tw.p, s->sms,
+                           s->st),
+            "rotation");
+    }
+    return 0;
 }
 
 int mset_rotate_volume_nd(mset_session *s, const float *vol_in, float *vol_out, int n1, int n2, int n3,
@@ -1362,9 +1427,10 @@ int mset_batch_iteration_setup_nd(mset_session *s, const mset_iter_args *a, int 
         return fail(MSET_E_ARG, "window minus volume sides must be even (centred padding)");
     if (a->use_tv && (!(a->tv_lambda > 0) || a->tv_iter < 0)) return fail(MSET_E_ARG, "bad TV parameters");
     const bool cubic = nv1 == nv2 && nv2 == nv3;
-    rc = cubic ? rot_prepare(s, nv1) : rot_prepare3(s, nv1, nv2, nv3);
-    if (rc) return rc;
     const int J = (int)s->tilts.size();
+    rc = cubic ? rot_prepare(s, nv1) : rot_prepare3(s, nv1, nv2, nv3);
+    if (!rc && cubic) rc = rot_prepare_group(s, nv1, J);
+    if (rc) return rc;
     const double v1[3] = {a->vec1[0], a->vec1[1], a->vec1[2]}, v2[3] = {a->vec2[0], a->vec2[1], a->vec2[2]},
                  v3[3] = {a->vec3[0], a->vec3[1], a->vec3[2]};
     s->plan_inv.resize(J);
@@ -1446,9 +1512,9 @@ static int record_phase(mset_session *s, int phase, bool with_tv = true, bool wi
     const size_t n2 = (size_t)n * n;
     if (phase == 2) goto update;
     // 1. beam-frame volumes V_j = pad(Func_inv_rot(rec, angles_j))
-    for (int j = 0; j < J; ++j) {
-        CKL(rotate_rec(s, s->plan_inv[j], s->rec.p, s->gvol.p), "rotation");
-        CKL(vol_pad(s->gvol.p, s->tilts[j].V.p, s->nv1, s->nv2, s->nv3, n, s->st), "pad");
+    {
+        const int rc = rec_to_tilts(s);
+        if (rc) return rc;
     }
     // 2. the batched pass over all positions of all tilts
     for (auto &t : s->tilts) {
@@ -1464,11 +1530,9 @@ static int record_phase(mset_session *s, int phase, bool with_tv = true, bool wi
         CKL(launch_positions(s->plan, s->method, s->adjoint, mode, la, s->grid_cache, s->st), "position kernel");
     }
     // 3. gradient back to the lab frame: sum_j Func_rot(G_j)
-    for (int j = 0; j < J; ++j) {
-        CKL(vol_slab_to_volume(s->tilts[j].grad.p, s->gvol.p, s->nv1, s->nv2, s->nv3, n, bvox, s->st),
-            "slab_to_volume");
-        CKL(rotate_rec(s, s->plan_fwd[j], s->gvol.p, s->gvol.p), "rotation");
-        CKL(vol_accumulate(s->gvol.p, s->gacc.p, V, j == 0, s->st), "accumulate");
+    {
+        const int rc = tilts_to_gacc(s, bvox);
+        if (rc) return rc;
     }
     if (phase == 1) return 0;
 update:
@@ -1569,10 +1633,8 @@ static int record_error_phase(mset_session *s) {
     const int n = s->n;
     const int nsg = s->method == MSET_MODE_SSET ? 1 : s->ns;
     const int bvox = s->method == MSET_MODE_SSET ? s->nz : s->b;
-    for (int j = 0; j < J; ++j) {
-        CKL(rotate_rec(s, s->plan_inv[j], s->rec.p, s->gvol.p), "rotation");
-        CKL(vol_pad(s->gvol.p, s->tilts[j].V.p, s->nv1, s->nv2, s->nv3, n, s->st), "pad");
-    }
+    const int rc = rec_to_tilts(s);
+    if (rc) return rc;
     CK(cudaMemsetAsync(s->err.p, 0, sizeof(double) * J, s->st));
     CKL(s->plan.ops->transmission(s->d_tilts.p, J, s->nz, bvox, nsg, s->sigma * s->dz, s->st), "transmission");
     CK(cudaMemsetAsync(s->counter.p, 0, sizeof(unsigned), s->st));

@@ -10,7 +10,10 @@
 // shared memory with the same radix passes as the multislice kernel; the
 // phase is the separable product ex(kx) ey(ky) computed in double per plane,
 // except where the reference's grid is zeroed (any Nyquist index), where it
-// is 1.  The complex volume stays L2-resident (16 MB at 128^3).
+// is 1.  The complex volume stays L2-resident (16 MB at 128^3).  A rotation
+// about a volume axis has shears of one coefficient (k_shear1) and one of none,
+// which is left out.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -30,84 +33,172 @@ __host__ __device__ inline int rot_grid_val(int i, int n, bool *nyq) {
     return *nyq ? 0 : (k + 1 - c);
 }
 
-template <int N>
-struct RotSmem {
-    static constexpr int EX = 0;  // float2 offsets after the field + twiddles
+// ---- volumes and their complex copies --------------------------------------
+// One complex work volume S per rotation job (blockIdx.y); thread t of a block
+// takes element t % n of row t / n, so no division depends on the element.
+struct Rows3 {
+    int n, rpb;  // volume edge, rows per block
+    __device__ __forceinline__ bool at(int row0, int &i1, int &i2, int &i3) const {
+        const int r = threadIdx.x / n;
+        const int row = row0 * rpb + r;
+        i1 = threadIdx.x % n;
+        i2 = row % n;
+        i3 = row / n;
+        return r < rpb && row < n * n;
+    }
+    // where element i of an axis lies after ifftshift (n even)
+    __device__ __forceinline__ int sh(int i) const { return i < n - n / 2 ? i + n / 2 : i - (n - n / 2); }
+    __device__ __forceinline__ long idx(int i1, int i2, int i3) const { return ((long)i3 * n + i2) * n + i1; }
 };
 
-// complex S = ifftshift(real vol)
-__global__ void k_rot_pre(const float *vol, float2 *S, int n) {
-    const long nn = (long)n * n, total = nn * n;
-    const int h = (n + 1) / 2;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int i3 = (int)(i / nn), i2 = (int)((i / n) % n), i1 = (int)(i % n);
-        const long o = (long)((i3 + h) % n) * nn + (long)((i2 + h) % n) * n + (i1 + h) % n;
-        S[o] = make_float2(vol[i], 0.f);
-    }
+// S_j = ifftshift(vol)
+__global__ void k_rot_load(const float *vol, float2 *S, Rows3 g, long stride) {
+    int i1, i2, i3;
+    if (g.at(blockIdx.x, i1, i2, i3))
+        S[blockIdx.y * stride + g.idx(g.sh(i1), g.sh(i2), g.sh(i3))] = make_float2(vol[g.idx(i1, i2, i3)], 0.f);
+}
+// out = fftshift(real(S))
+__global__ void k_rot_store(const float2 *S, float *out, Rows3 g) {
+    int i1, i2, i3;
+    if (g.at(blockIdx.x, i1, i2, i3)) out[g.idx(i1, i2, i3)] = S[g.idx(g.sh(i1), g.sh(i2), g.sh(i3))].x;
+}
+struct RotPtrs {
+    void *p[kRotJobs];
+};
+// S_j = ifftshift of a tilt's slab gradient (FP64 [ns][w][w]), each slab on its
+// b voxels, cropped to the volume
+__global__ void k_rot_load_slabs(RotPtrs grads, float2 *S, Rows3 g, long stride, int w, int b) {
+    int i1, i2, i3;
+    if (!g.at(blockIdx.x, i1, i2, i3)) return;
+    const double *G = static_cast<const double *>(grads.p[blockIdx.y]);
+    const int o = (w - g.n) / 2;
+    S[blockIdx.y * stride + g.idx(g.sh(i1), g.sh(i2), g.sh(i3))] =
+        make_float2((float)G[((long)(i3 / b) * w + i2 + o) * w + i1 + o], 0.f);
+}
+// V_j [n][w][w] = fftshift(real(S_j)) laterally centred in the window, zero around it
+__global__ void k_rot_store_window(const float2 *S, RotPtrs vols, Rows3 g, long stride, int w) {
+    const int rows = blockDim.x / w, r = threadIdx.x / w, x = threadIdx.x % w;
+    const int row = blockIdx.x * rows + r, y = row % w, z = row / w, o = (w - g.n) / 2;
+    if (r >= rows || z >= g.n) return;
+    const int i1 = x - o, i2 = y - o;
+    const bool in = i1 >= 0 && i1 < g.n && i2 >= 0 && i2 < g.n;
+    static_cast<float *>(vols.p[blockIdx.y])[((long)z * w + y) * w + x] =
+        in ? S[blockIdx.y * stride + g.idx(g.sh(i1), g.sh(i2), g.sh(z))].x : 0.f;
+}
+// acc (+)= sum over jobs, in their order, of fftshift(real(S_j)), FP64
+__global__ void k_rot_accumulate(const float2 *S, double *acc, Rows3 g, long stride, int jobs, int zero) {
+    int i1, i2, i3;
+    if (!g.at(blockIdx.x, i1, i2, i3)) return;
+    const long o = g.idx(i1, i2, i3), i = g.idx(g.sh(i1), g.sh(i2), g.sh(i3));
+    double a = zero ? 0.0 : acc[o];
+    for (int j = 0; j < jobs; ++j) a += (double)S[j * stride + i].x;
+    acc[o] = a;
 }
 
-// out = fftshift(real(S)); out[(i + floor(n/2)) mod n] = S[i]
-__global__ void k_rot_post(const float2 *S, float *out, int n) {
-    const long nn = (long)n * n, total = nn * n;
-    const int h = n / 2;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int i3 = (int)(i / nn), i2 = (int)((i / n) % n), i1 = (int)(i % n);
-        const long o = (long)((i3 + h) % n) * nn + (long)((i2 + h) % n) * n + (i1 + h) % n;
-        out[o] = S[i].x;
-    }
-}
-
+// ---- shears ------------------------------------------------------------------
 // One shear along MATLAB dimension `dim` (1: x fastest, 2: y, 3: z) with
-// coefficients (ca, cb) for every plane; REAL keeps only the real part
-// (the fourth shear of a sub-step, Func_rotate_3Dvol_ROTmat_FourierShear.m:121, 126).
-template <class G, bool REAL>
-__global__ void __launch_bounds__(G::NT, 1) k_shear(float2 *S, const float2 *twn, int dim, double ca, double cb) {
-    constexpr int N = G::N, R1 = G::R1, R2 = G::R2;
+// coefficients (ca, cb); real: keep only the real part (the fourth shear of a
+// sub-step, Func_rotate_3Dvol_ROTmat_FourierShear.m:121, 126).
+struct ShearJob {
+    float2 *S;
+    double ca, cb;
+    int dim, real;
+};
+struct ShearJobs {
+    ShearJob j[kRotJobs];
+};
+
+// A plane between global memory (rows at stride sw, elements at su) and shared
+// memory; the loads are asynchronous (plane_wait).  Lanes run along the
+// contiguous axis: along u, or 4 rows by 8 elements, which covers 32-byte
+// sectors with two-way bank conflicts.
+template <class G>
+__device__ __forceinline__ void plane_pos(int i, bool across, int &r, int &u) {
+    constexpr int N = G::N;
+    if (across) {
+        const int q = i / (4 * N), m = i % (4 * N);
+        r = 4 * q + m % 4;
+        u = m / 4;
+    } else {
+        r = i / N;
+        u = i % N;
+    }
+}
+template <class G>
+__device__ __forceinline__ void plane_load(float2 *buf, const float2 *p, long su, long sw) {
+    const int yb = G::ybase();
+    const bool across = sw == 1 && G::CL == 1;
+    for (int i = threadIdx.x; i < G::ROWS * G::N; i += G::NT) {
+        int r, u;
+        plane_pos<G>(i, across, r, u);
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(buf + G::at(r, u));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(p + (long)G::gy(yb, r) * sw + (long)u * su)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void plane_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <class G>
+__device__ __forceinline__ void plane_store(const float2 *buf, float2 *p, long su, long sw, bool real) {
+    const int yb = G::ybase();
+    const bool across = sw == 1 && G::CL == 1;
+    for (int i = threadIdx.x; i < G::ROWS * G::N; i += G::NT) {
+        int r, u;
+        plane_pos<G>(i, across, r, u);
+        float2 v = buf[G::at(r, u)];
+        if (real) v.y = 0.f;
+        p[(long)G::gy(yb, r) * sw + (long)u * su] = v;
+    }
+}
+// a plane the shear does not move: only the fourth shear's real() acts
+template <class G>
+__device__ __forceinline__ void plane_keep(float2 *p, long su, long sw, bool real) {
+    const int yb = G::ybase();
+    if (real)
+        for (int i = threadIdx.x; i < G::ROWS * G::N; i += G::NT)
+            p[(long)G::gy(yb, i / G::N) * sw + (long)(i % G::N) * su].y = 0.f;
+}
+
+// strides of the plane axes x' (transformed along shared-memory rows) and y'
+// and of the shear axis
+template <int N>
+__device__ __forceinline__ void plane_strides(int dim, long &sx, long &sy, long &sc) {
+    const long nn = (long)N * N;
+    sx = dim == 1 ? N : 1;
+    sy = dim == 3 ? N : nn;
+    sc = dim == 1 ? 1 : dim == 2 ? N : nn;
+}
+
+template <class G>
+__global__ void __launch_bounds__(G::NT, 1) k_shear(ShearJobs jobs, const float2 *twn) {
+    constexpr int N = G::N, R1 = G::R1;
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm;
     float2 *tw = buf + G::FIELD;
     float2 *ex = tw + N;
     float2 *ey = ex + N;
     __shared__ int nyx[N], nyy[N];
+    const ShearJob &job = jobs.j[blockIdx.y];
+    const bool real = job.real != 0;
     for (int i = threadIdx.x; i < N; i += G::NT) tw[i] = twn[i];
-    const long nn = (long)N * N;
-    // plane axes: x' (fast, shared-memory rows) and y' (slow)
     long sx, sy, sc;
-    if (dim == 1) {
-        sx = N; sy = nn; sc = 1;      // plane (i2, i3) at fixed i1
-    } else if (dim == 2) {
-        sx = 1; sy = nn; sc = N;      // plane (i1, i3) at fixed i2
-    } else {
-        sx = 1; sy = N; sc = nn;      // plane (i1, i2) at fixed i3
-    }
+    plane_strides<N>(job.dim, sx, sy, sc);
     const float inv = 1.0f / (float)(N * N);
     // one plane per CTA, or per cluster when the plane is split by rows
-    const int yb = G::ybase();
     sync_all<G>();  // (cluster) every CTA has started before any remote access
     for (int c = blockIdx.x / G::CL; c < N; c += gridDim.x / G::CL) {
         bool qc;
         const int gc = rot_grid_val(c, N, &qc);
-        if (qc) {
-            // the reference's grids are zero on this plane: no shift; only the
-            // fourth shear's real() acts
-            if (REAL) {
-                for (int i = threadIdx.x; i < G::ROWS * N; i += G::NT) {
-                    float2 *p = S + (long)c * sc + (long)G::gy(yb, i / N) * sy + (long)(i % N) * sx;
-                    p->y = 0.f;
-                }
-            }
+        float2 *p = job.S + (long)c * sc;
+        if (gc == 0) {  // the grids are zero on the Nyquist plane too
+            plane_keep<G>(p, sx, sy, real);
             sync_all<G>();
             continue;
         }
-        // per-plane phase factors (double): phase = 2 pi gc (cx gx(kx) + cy gy(ky)) / N
-        double cx, cy;
-        if (dim == 1) {
-            cx = ca; cy = cb;  // a with n2 (x'), b with n3 (y')
-        } else if (dim == 2) {
-            cx = cb; cy = ca;  // b with n1 (x'), a with n3 (y')
-        } else {
-            cx = ca; cy = cb;  // a with n1 (x'), b with n2 (y')
-        }
+        plane_load<G>(buf, p, sx, sy);
+        // per-plane phase factors (double): phase = 2 pi gc (cx gx(kx) + cy gy(ky)) / N;
+        // dim 1: a with n2 (x'), b with n3 (y'); 2: b with n1, a with n3; 3: a with n1, b with n2
+        const double cx = job.dim == 2 ? job.cb : job.ca, cy = job.dim == 2 ? job.ca : job.cb;
         for (int L = threadIdx.x; L < N; L += G::NT) {
             const int k = G::scr(L);
             bool q;
@@ -120,10 +211,7 @@ __global__ void __launch_bounds__(G::NT, 1) k_shear(float2 *S, const float2 *twn
             ey[L] = make_float2((float)co, (float)s);
             nyy[L] = q;
         }
-        for (int i = threadIdx.x; i < G::ROWS * N; i += G::NT) {
-            const int yy = i / N, xx = i % N;
-            buf[G::at(yy, xx)] = S[(long)c * sc + (long)G::gy(yb, yy) * sy + (long)xx * sx];
-        }
+        plane_wait();
         __syncthreads();
         row_passA<G, 0, -1>(buf, tw, NoOp{});
         sync_rows();
@@ -147,33 +235,122 @@ __global__ void __launch_bounds__(G::NT, 1) k_shear(float2 *S, const float2 *twn
         sync_rows();
         row_passA<G, +1, 0>(buf, tw, NoOp{});
         __syncthreads();
-        for (int i = threadIdx.x; i < G::ROWS * N; i += G::NT) {
-            const int yy = i / N, xx = i % N;
-            float2 v = buf[G::at(yy, xx)];
-            if (REAL) v.y = 0.f;
-            S[(long)c * sc + (long)G::gy(yb, yy) * sy + (long)xx * sx] = v;
-        }
+        plane_store<G>(buf, p, sx, sy, real);
         sync_all<G>();
-        (void)R2;
     }
 }
 
+// A shear with one coefficient (a rotation about a volume axis has only such
+// ones): the plane's rows along the other axis u move on their own, except that
+// the spectrum's Nyquist line across the rows stays (its grid is zeroed), so
+//   out(k, w) = e(k) S(k, w) + (1 - e(k)) (-1)^w c(k),
+//   c(k) = sum_w (-1)^w S(k, w) / N
+// with e the phase along u: one transform along u each way and one alternating
+// column sum, 4 passes over the plane instead of 7.
 template <class G>
-static size_t shear_smem() {
-    return sizeof(float2) * ((size_t)G::FIELD + 3 * G::N);
+constexpr int kSumParts = G::NT / G::N > 4 ? 4 : G::NT / G::N;
+template <class G>
+__global__ void __launch_bounds__(G::NT, 1) k_shear1(ShearJobs jobs, const float2 *twn) {
+    constexpr int N = G::N, R1 = G::R1, R2 = G::R2, PARTS = kSumParts<G>;
+    static_assert(PARTS >= 1, "a thread per column");
+    extern __shared__ __align__(16) float2 sm[];
+    float2 *buf = sm;
+    float2 *tw = buf + G::FIELD;
+    float2 *f = tw + N, *h = f + N, *part = h + N;
+    const ShearJob &job = jobs.j[blockIdx.y];
+    const bool real = job.real != 0;
+    long sx, sy, sc;
+    plane_strides<N>(job.dim, sx, sy, sc);
+    // u: the axis of the one coefficient
+    const double cx = job.dim == 2 ? job.cb : job.ca, cy = job.dim == 2 ? job.ca : job.cb;
+    const long su = cy == 0.0 ? sx : sy, sw = cy == 0.0 ? sy : sx;
+    const double cu = cy == 0.0 ? cx : cy;
+    const float inv = 1.0f / (float)N;
+    const int c = blockIdx.x, gc = [&] {
+        bool q;
+        return rot_grid_val(c, N, &q);
+    }();
+    float2 *p = job.S + (long)c * sc;
+    if (gc == 0 || cu == 0.0) {
+        plane_keep<G>(p, su, sw, real);
+        return;
+    }
+    plane_load<G>(buf, p, su, sw);
+    for (int L = threadIdx.x; L < N; L += G::NT) {
+        tw[L] = twn[L];
+        bool q;
+        const int g = rot_grid_val(G::scr(L), N, &q);
+        double s, co;
+        sincospi(2.0 * (double)gc * cu * (double)g / (double)N, &s, &co);  // the Nyquist grid value is 0
+        f[L] = make_float2((float)co, (float)s);
+    }
+    plane_wait();
+    __syncthreads();
+    row_passA<G, 0, -1>(buf, tw, NoOp{});
+    sync_rows();
+    row_passB<G, -1>(buf);
+    __syncthreads();
+    if (threadIdx.x < PARTS * N) {
+        const int L = threadIdx.x % N, w0 = threadIdx.x / N;
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int w = w0; w < N; w += PARTS) {
+            const float2 v = buf[G::at(w, L)];
+            acc = (w & 1) ? csub(acc, v) : cadd(acc, v);
+        }
+        part[w0 * N + L] = acc;
+    }
+    __syncthreads();
+    for (int L = threadIdx.x; L < N; L += G::NT) {
+        float2 acc = part[L];
+#pragma unroll
+        for (int q = 1; q < PARTS; ++q) acc = cadd(acc, part[q * N + L]);
+        const float2 e = f[L];
+        h[L] = cscale(cmul(make_float2(1.f - e.x, -e.y), acc), inv * inv);
+        f[L] = cscale(e, inv);
+    }
+    __syncthreads();
+    // inverse row pass B with the phase
+    using O = Own<G>;
+    const int y0 = O::warp() * O::RPW;
+#pragma unroll 1
+    for (int tau = O::lane(); tau < O::RPW * R2; tau += 32) {
+        const int k2 = tau % R2, y = y0 + tau / R2;
+        float2 *b = buf + y * G::S + G::xb0(k2);
+        float2 v[R1];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+            const float2 t = cmul(b[G::xb(k2, j)], f[R1 * k2 + j]), n = h[R1 * k2 + j];
+            v[j] = (y & 1) ? csub(t, n) : cadd(t, n);
+        }
+        DFT<R1, +1>::run(v);
+#pragma unroll
+        for (int j = 0; j < R1; ++j) b[G::xb(k2, j)] = v[j];
+    }
+    sync_rows();
+    const bool direct = su == 1;  // rows contiguous in memory: straight from pass A
+    row_passA<G, +1, 0>(buf, tw, [&](int y, int n1, float2 *v) {
+        if (direct)
+#pragma unroll
+            for (int j = 0; j < R2; ++j)
+                p[(long)y * sw + n1 + R1 * j] = make_float2(v[j].x, real ? 0.f : v[j].y);
+    });
+    if (direct) return;
+    __syncthreads();
+    plane_store<G>(buf, p, su, sw, real);
 }
 
-template <class G, bool REAL>
-static int launch_shear_k(float2 *S, const float2 *twn, int dim, double a, double b, int grid, cudaStream_t st) {
-    auto k = k_shear<G, REAL>;
-    const size_t sm = shear_smem<G>();
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return (int)e;
+template <class G>
+static int launch_shear(const ShearJobs &jobs, int count, bool one, const float2 *twn, int sms, cudaStream_t st) {
     if constexpr (G::CL > 1) {
+        auto k = k_shear<G>;
+        const size_t smem = sizeof(float2) * ((size_t)G::FIELD + 3 * G::N);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
+        cfg.gridDim = dim3(std::min(G::N, sms / G::CL) * G::CL, count);
         cfg.blockDim = dim3(G::NT);
-        cfg.dynamicSmemBytes = sm;
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -182,20 +359,16 @@ static int launch_shear_k(float2 *S, const float2 *twn, int dim, double a, doubl
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        return (int)cudaLaunchKernelEx(&cfg, k, S, twn, dim, a, b);
+        return (int)cudaLaunchKernelEx(&cfg, k, jobs, twn);
     } else {
-        k<<<grid, G::NT, sm, st>>>(S, twn, dim, a, b);
+        auto k = one ? k_shear1<G> : k_shear<G>;
+        const size_t smem = sizeof(float2) * ((size_t)G::FIELD + (one ? 3 + kSumParts<G> : 3) * G::N);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        // planes in flight: one per CTA (k_shear1: one plane per CTA in all)
+        k<<<dim3(one ? G::N : std::min(G::N, sms), count), G::NT, smem, st>>>(jobs, twn);
         return (int)cudaGetLastError();
     }
-}
-
-template <class G>
-static int launch_shear(float2 *S, const float2 *twn, int dim, double a, double b, bool real, int sms,
-                        cudaStream_t st) {
-    // planes in flight: one per CTA, or one per cluster of CL CTAs
-    const int grid = std::min(G::N, sms / G::CL) * G::CL;
-    return real ? launch_shear_k<G, true>(S, twn, dim, a, b, grid, st)
-                : launch_shear_k<G, false>(S, twn, dim, a, b, grid, st);
 }
 
 #define MSET_ROT_GEOS(X) X(24, 8, 64) X(32, 8, 128) X(48, 16, 192) X(64, 8, 256) X(96, 16, 384) X(128, 16, 512) X(160, 16, 640)
@@ -218,15 +391,18 @@ int rot_r1(int n) {
     return n == 256 ? RotGeo256::R1 : 0;
 }
 
-static int shear(int n, float2 *S, const float2 *twn, int dim, double a, double b, bool real, int sms,
-                 cudaStream_t st) {
+static int shear(int n, const ShearJobs &jobs, int count, bool one, const float2 *twn, int sms, cudaStream_t st) {
 #define X(N_, R1_, NT_) \
-    if (n == N_) return launch_shear<Geo<N_, R1_, NT_>>(S, twn, dim, a, b, real, sms, st);
+    if (n == N_) return launch_shear<Geo<N_, R1_, NT_>>(jobs, count, one, twn, sms, st);
     MSET_ROT_GEOS(X)
 #undef X
-    if (n == 256) return launch_shear<RotGeo256>(S, twn, dim, a, b, real, sms, st);
+    if (n == 256) return launch_shear<RotGeo256>(jobs, count, one, twn, sms, st);
     return (int)cudaErrorInvalidValue;
 }
+
+// a coefficient whose largest phase, pi (n / 2) |c| rad, is under 2^-30, far
+// below what FP32 phase factors resolve
+static bool no_shear(double c, int n) { return M_PI * 0.5 * n * std::fabs(c) < 9.3e-10; }
 
 // ---------------------------------------------------------------------------
 // volumes of any shape n1 x n2 x n3: every shear as batched 1D transforms
@@ -490,6 +666,10 @@ int rot_apply3(const RotPlan &pl, int n1, int n2, int n3, const float *vol, floa
     if (rc) return rc;
     for (int s = 0; s < pl.num_step; ++s)
         for (int k = 0; k < 4; ++k) {
+            // (only the fourth shear takes the real part)
+            if (k < 3 && no_shear(pl.a[k], std::max(n1, std::max(n2, n3))) &&
+                no_shear(pl.b[k], std::max(n1, std::max(n2, n3))))
+                continue;
             rc = shear_lines(n, S, pl.dim[k], pl.a[k], pl.b[k], k == 3, sms, st);
             if (rc) return rc;
         }
@@ -650,6 +830,41 @@ int rot_twiddles(int n, std::vector<float2> &h) {
     return 0;
 }
 
+namespace {
+Rows3 rows3_of(int n) { return Rows3{n, 256 / n}; }
+dim3 rows3_grid(const Rows3 &g, int jobs) { return dim3((g.n * g.n + g.rpb - 1) / g.rpb, jobs); }
+
+// every shear of `count` rotations, each on its work volume, step by step:
+// the rotations' shears of one step share a launch (small volumes leave most of
+// the chip idle)
+int shear_all(const RotPlan *const *plans, int count, int n, float2 *S, const float2 *twn, int sms, cudaStream_t st) {
+    const long stride = (long)n * n * n;
+    int steps = 0;
+    for (int j = 0; j < count; ++j)
+        if (plans[j]->active) steps = std::max(steps, plans[j]->num_step);
+    for (int s = 0; s < steps; ++s)
+        for (int k = 0; k < 4; ++k) {
+            ShearJobs one, two;
+            int n1 = 0, n2 = 0;
+            for (int j = 0; j < count; ++j) {
+                const RotPlan &pl = *plans[j];
+                if (!pl.active || s >= pl.num_step) continue;
+                ShearJob job{S + j * stride, no_shear(pl.a[k], n) ? 0.0 : pl.a[k], no_shear(pl.b[k], n) ? 0.0 : pl.b[k],
+                             pl.dim[k], k == 3};
+                const bool none = job.ca == 0.0 && job.cb == 0.0;
+                if (none && k < 3) continue;  // moves nothing
+                // (256: planes over a cluster, both kinds in k_shear)
+                if ((job.ca == 0.0 || job.cb == 0.0) && n != 256) one.j[n1++] = job;
+                else two.j[n2++] = job;
+            }
+            int rc = n1 ? shear(n, one, n1, true, twn, sms, st) : 0;
+            if (!rc && n2) rc = shear(n, two, n2, false, twn, sms, st);
+            if (rc) return rc;
+        }
+    return 0;
+}
+}  // namespace
+
 // out = rotation of vol (both device [n][n][n] float, may alias), S = n^3 complex work
 int rot_apply(const RotPlan &pl, int n, const float *vol, float *out, float2 *S, const float2 *twn, int sms,
               cudaStream_t st) {
@@ -661,16 +876,46 @@ int rot_apply(const RotPlan &pl, int n, const float *vol, float *out, float2 *S,
         }
         return 0;
     }
-    const int g = (int)std::min<long>((total + 255) / 256, (long)sms * 8);
-    k_rot_pre<<<g, 256, 0, st>>>(vol, S, n);
+    const Rows3 g = rows3_of(n);
+    const RotPlan *one = &pl;
+    k_rot_load<<<rows3_grid(g, 1), 256, 0, st>>>(vol, S, g, total);
     int rc = (int)cudaGetLastError();
+    if (!rc) rc = shear_all(&one, 1, n, S, twn, sms, st);
     if (rc) return rc;
-    for (int s = 0; s < pl.num_step; ++s)
-        for (int k = 0; k < 4; ++k) {
-            rc = shear(n, S, twn, pl.dim[k], pl.a[k], pl.b[k], k == 3, sms, st);
-            if (rc) return rc;
-        }
-    k_rot_post<<<g, 256, 0, st>>>(S, out, n);
+    k_rot_store<<<rows3_grid(g, 1), 256, 0, st>>>(S, out, g);
+    return (int)cudaGetLastError();
+}
+
+// the beam-frame volumes of `count` tilts: V_j [n][w][w] = rotation of vol by
+// plan j, laterally centred in the window
+int rot_to_windows(const RotPlan *const *plans, int count, int n, const float *vol, float *const *V, int w, float2 *S,
+                   const float2 *twn, int sms, cudaStream_t st) {
+    const Rows3 g = rows3_of(n);
+    const long stride = (long)n * n * n;
+    RotPtrs out{};
+    for (int j = 0; j < count; ++j) out.p[j] = V[j];
+    k_rot_load<<<rows3_grid(g, count), 256, 0, st>>>(vol, S, g, stride);
+    int rc = (int)cudaGetLastError();
+    if (!rc) rc = shear_all(plans, count, n, S, twn, sms, st);
+    if (rc) return rc;
+    const int rows = 256 / w;
+    k_rot_store_window<<<dim3((n * w + rows - 1) / rows, count), 256, 0, st>>>(S, out, g, stride, w);
+    return (int)cudaGetLastError();
+}
+
+// acc (+)= sum over `count` tilts of the rotation by plan j of the slab
+// gradient G_j (FP64 [ns][w][w], each slab on its b voxels)
+int rot_accumulate(const RotPlan *const *plans, int count, int n, const double *const *G, int w, int b, double *acc,
+                   bool zero, float2 *S, const float2 *twn, int sms, cudaStream_t st) {
+    const Rows3 g = rows3_of(n);
+    const long stride = (long)n * n * n;
+    RotPtrs in{};
+    for (int j = 0; j < count; ++j) in.p[j] = const_cast<double *>(G[j]);
+    k_rot_load_slabs<<<rows3_grid(g, count), 256, 0, st>>>(in, S, g, stride, w, b);
+    int rc = (int)cudaGetLastError();
+    if (!rc) rc = shear_all(plans, count, n, S, twn, sms, st);
+    if (rc) return rc;
+    k_rot_accumulate<<<rows3_grid(g, 1), 256, 0, st>>>(S, acc, g, stride, count, zero ? 1 : 0);
     return (int)cudaGetLastError();
 }
 

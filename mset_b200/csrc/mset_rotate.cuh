@@ -21,6 +21,13 @@ int rot_twiddles(int n, std::vector<float2> &h);
 // out = rotation of vol (device, [n][n][n]); S: n^3 complex work buffer
 int rot_apply(const RotPlan &pl, int n, const float *vol, float *out, float2 *S, const float2 *twn, int sms,
               cudaStream_t st);
+// several rotations of cubic volumes at once, at most kRotJobs; S: count n^3
+// complex work volumes (see mset_rotate.cu)
+constexpr int kRotJobs = 16;
+int rot_to_windows(const RotPlan *const *plans, int count, int n, const float *vol, float *const *V, int w, float2 *S,
+                   const float2 *twn, int sms, cudaStream_t st);
+int rot_accumulate(const RotPlan *const *plans, int count, int n, const double *const *G, int w, int b, double *acc,
+                   bool zero, float2 *S, const float2 *twn, int sms, cudaStream_t st);
 // any shape [n3][n2][n1] (every side a supported line length): each shear as
 // batched 1D transforms; S: n1 n2 n3 complex work buffer
 bool rot_line_supported(int n);
