@@ -34,65 +34,99 @@ __host__ __device__ inline int rot_grid_val(int i, int n, bool *nyq) {
 }
 
 // ---- volumes and their complex copies --------------------------------------
-// One complex work volume S per rotation job (blockIdx.y); thread t of a block
-// takes element t % n of row t / n, so no division depends on the element.
-struct Rows3 {
-    int n, rpb;  // volume edge, rows per block
-    __device__ __forceinline__ bool at(int row0, int &i1, int &i2, int &i3) const {
-        const int r = threadIdx.x / n;
-        const int row = row0 * rpb + r;
-        i1 = threadIdx.x % n;
-        i2 = row % n;
-        i3 = row / n;
-        return r < rpb && row < n * n;
-    }
+// One complex work volume S per rotation (blockIdx.y).  S keeps the volume's
+// order (x fastest) or x swapped with the axis `f` (1: y, 2: z) that no shear
+// of the rotation runs along, so that every plane holds its fastest axis: a
+// plane of fixed x in the volume's order is read and written in 8-byte pieces
+// of 32-byte sectors (43 us per shear at 128^3 against 20).
+struct Axes {
+    int n;
     // where element i of an axis lies after ifftshift (n even)
     __device__ __forceinline__ int sh(int i) const { return i < n - n / 2 ? i + n / 2 : i - (n - n / 2); }
     __device__ __forceinline__ long idx(int i1, int i2, int i3) const { return ((long)i3 * n + i2) * n + i1; }
+    // index in S of the ifftshifted element
+    __device__ __forceinline__ long in_s(int f, int i1, int i2, int i3) const {
+        const int a = sh(i1), b = sh(i2), c = sh(i3);
+        return f == 0 ? idx(a, b, c) : f == 1 ? idx(b, a, c) : idx(c, b, a);
+    }
 };
-
-// S_j = ifftshift(vol)
-__global__ void k_rot_load(const float *vol, float2 *S, Rows3 g, long stride) {
-    int i1, i2, i3;
-    if (g.at(blockIdx.x, i1, i2, i3))
-        S[blockIdx.y * stride + g.idx(g.sh(i1), g.sh(i2), g.sh(i3))] = make_float2(vol[g.idx(i1, i2, i3)], 0.f);
-}
-// out = fftshift(real(S))
-__global__ void k_rot_store(const float2 *S, float *out, Rows3 g) {
-    int i1, i2, i3;
-    if (g.at(blockIdx.x, i1, i2, i3)) out[g.idx(i1, i2, i3)] = S[g.idx(g.sh(i1), g.sh(i2), g.sh(i3))].x;
-}
 struct RotPtrs {
     void *p[kRotJobs];
+    int f[kRotJobs];  // fastest axis of S_j
 };
-// S_j = ifftshift of a tilt's slab gradient (FP64 [ns][w][w]), each slab on its
-// b voxels, cropped to the volume
-__global__ void k_rot_load_slabs(RotPtrs grads, float2 *S, Rows3 g, long stride, int w, int b) {
-    int i1, i2, i3;
-    if (!g.at(blockIdx.x, i1, i2, i3)) return;
-    const double *G = static_cast<const double *>(grads.p[blockIdx.y]);
-    const int o = (w - g.n) / 2;
-    S[blockIdx.y * stride + g.idx(g.sh(i1), g.sh(i2), g.sh(i3))] =
-        make_float2((float)G[((long)(i3 / b) * w + i2 + o) * w + i1 + o], 0.f);
+constexpr int kTile = 32;
+// A block's tile of 32 x by 32 of the axis g (y, or z when S has z fastest) at
+// one place of the third axis; body(i1, i2, i3, tile element) for every
+// element, the lanes along x (along_x) or along g
+template <class Body>
+__device__ __forceinline__ void for_tile(int n, int g, bool along_x, float (*tile)[kTile + 1], Body &&body) {
+    const int nt = (n + kTile - 1) / kTile;
+    const int tx = blockIdx.x % nt, tg = blockIdx.x / nt % nt, o = blockIdx.x / (nt * nt);
+    for (int r = threadIdx.y; r < kTile; r += blockDim.y) {
+        const int dx = along_x ? threadIdx.x : r, dg = along_x ? r : threadIdx.x;
+        const int i1 = tx * kTile + dx, ig = tg * kTile + dg;
+        if (i1 < n && ig < n) body(i1, g == 1 ? ig : o, g == 1 ? o : ig, tile[dg][dx]);
+    }
 }
-// V_j [n][w][w] = fftshift(real(S_j)) laterally centred in the window, zero around it
-__global__ void k_rot_store_window(const float2 *S, RotPtrs vols, Rows3 g, long stride, int w) {
-    const int rows = blockDim.x / w, r = threadIdx.x / w, x = threadIdx.x % w;
-    const int row = blockIdx.x * rows + r, y = row % w, z = row / w, o = (w - g.n) / 2;
-    if (r >= rows || z >= g.n) return;
-    const int i1 = x - o, i2 = y - o;
-    const bool in = i1 >= 0 && i1 < g.n && i2 >= 0 && i2 < g.n;
-    static_cast<float *>(vols.p[blockIdx.y])[((long)z * w + y) * w + x] =
-        in ? S[blockIdx.y * stride + g.idx(g.sh(i1), g.sh(i2), g.sh(z))].x : 0.f;
+inline dim3 tile_grid(int n, int jobs) {
+    const int nt = (n + kTile - 1) / kTile;
+    return dim3(nt * nt * n, jobs);
 }
-// acc (+)= sum over jobs, in their order, of fftshift(real(S_j)), FP64
-__global__ void k_rot_accumulate(const float2 *S, double *acc, Rows3 g, long stride, int jobs, int zero) {
-    int i1, i2, i3;
-    if (!g.at(blockIdx.x, i1, i2, i3)) return;
-    const long o = g.idx(i1, i2, i3), i = g.idx(g.sh(i1), g.sh(i2), g.sh(i3));
-    double a = zero ? 0.0 : acc[o];
-    for (int j = 0; j < jobs; ++j) a += (double)S[j * stride + i].x;
-    acc[o] = a;
+__device__ __forceinline__ int tile_axis(int f) { return f == 2 ? 2 : 1; }
+
+// S_j = ifftshift of vol (grads null), or of a tilt's slab gradient (FP64
+// [ns][w][w]), each slab on its b voxels, cropped to the volume
+template <bool SLABS>
+__global__ void __launch_bounds__(256) k_rot_load(const float *vol, RotPtrs j, float2 *S, Axes x, long stride, int w,
+                                                  int b) {
+    __shared__ float tile[kTile][kTile + 1];
+    const int f = j.f[blockIdx.y], g = tile_axis(f), o = (w - x.n) / 2;
+    const double *G = static_cast<const double *>(j.p[blockIdx.y]);
+    for_tile(x.n, g, true, tile, [&](int i1, int i2, int i3, float &t) {
+        if constexpr (SLABS) t = (float)G[((long)(i3 / b) * w + i2 + o) * w + i1 + o];
+        else t = vol[x.idx(i1, i2, i3)];
+    });
+    __syncthreads();
+    for_tile(x.n, g, f == 0, tile, [&](int i1, int i2, int i3, float &t) {
+        S[blockIdx.y * stride + x.in_s(f, i1, i2, i3)] = make_float2(t, 0.f);
+    });
+}
+// out = fftshift(real(S))
+__global__ void __launch_bounds__(256) k_rot_store(const float2 *S, float *out, Axes x, int f) {
+    __shared__ float tile[kTile][kTile + 1];
+    const int g = tile_axis(f);
+    for_tile(x.n, g, f == 0, tile, [&](int i1, int i2, int i3, float &t) { t = S[x.in_s(f, i1, i2, i3)].x; });
+    __syncthreads();
+    for_tile(x.n, g, true, tile, [&](int i1, int i2, int i3, float &t) { out[x.idx(i1, i2, i3)] = t; });
+}
+// V_j [n][w][w] = fftshift(real(S_j)) laterally centred in the window (the
+// caller zeroes what lies around it)
+__global__ void __launch_bounds__(256) k_rot_store_window(const float2 *S, RotPtrs j, Axes x, long stride, int w) {
+    __shared__ float tile[kTile][kTile + 1];
+    const int f = j.f[blockIdx.y], g = tile_axis(f), o = (w - x.n) / 2;
+    float *V = static_cast<float *>(j.p[blockIdx.y]);
+    for_tile(x.n, g, f == 0, tile,
+             [&](int i1, int i2, int i3, float &t) { t = S[blockIdx.y * stride + x.in_s(f, i1, i2, i3)].x; });
+    __syncthreads();
+    for_tile(x.n, g, true, tile,
+             [&](int i1, int i2, int i3, float &t) { V[((long)i3 * w + i2 + o) * w + i1 + o] = t; });
+}
+// acc (+)= sum over the jobs, in their order, of fftshift(real(S_j)), FP64
+__global__ void __launch_bounds__(256) k_rot_accumulate(const float2 *S, double *acc, RotPtrs j, Axes x, long stride,
+                                                        int jobs, int zero) {
+    __shared__ float tile[kTile][kTile + 1];
+    // every job's tile is the same voxels: they share one tile axis (shear_all)
+    const int g = tile_axis(j.f[0]);
+    for (int k = 0; k < jobs; ++k) {
+        const int f = j.f[k];
+        __syncthreads();
+        for_tile(x.n, g, f == 0, tile, [&](int i1, int i2, int i3, float &t) { t = S[k * stride + x.in_s(f, i1, i2, i3)].x; });
+        __syncthreads();
+        for_tile(x.n, g, true, tile, [&](int i1, int i2, int i3, float &t) {
+            const long i = x.idx(i1, i2, i3);
+            acc[i] = (zero && k == 0 ? 0.0 : acc[i]) + (double)t;
+        });
+    }
 }
 
 // ---- shears ------------------------------------------------------------------
@@ -101,8 +135,9 @@ __global__ void k_rot_accumulate(const float2 *S, double *acc, Rows3 g, long str
 // sub-step, Func_rotate_3Dvol_ROTmat_FourierShear.m:121, 126).
 struct ShearJob {
     float2 *S;
-    double ca, cb;
-    int dim, real;
+    double cx, cy;   // coefficients of the plane axes x' and y'
+    int sx, sy, sc;  // strides of x' (the shared-memory rows), y' and the shear axis
+    int real;
 };
 struct ShearJobs {
     ShearJob j[kRotJobs];
@@ -159,16 +194,6 @@ __device__ __forceinline__ void plane_keep(float2 *p, long su, long sw, bool rea
             p[(long)G::gy(yb, i / G::N) * sw + (long)(i % G::N) * su].y = 0.f;
 }
 
-// strides of the plane axes x' (transformed along shared-memory rows) and y'
-// and of the shear axis
-template <int N>
-__device__ __forceinline__ void plane_strides(int dim, long &sx, long &sy, long &sc) {
-    const long nn = (long)N * N;
-    sx = dim == 1 ? N : 1;
-    sy = dim == 3 ? N : nn;
-    sc = dim == 1 ? 1 : dim == 2 ? N : nn;
-}
-
 template <class G>
 __global__ void __launch_bounds__(G::NT, 1) k_shear(ShearJobs jobs, const float2 *twn) {
     constexpr int N = G::N, R1 = G::R1;
@@ -181,8 +206,7 @@ __global__ void __launch_bounds__(G::NT, 1) k_shear(ShearJobs jobs, const float2
     const ShearJob &job = jobs.j[blockIdx.y];
     const bool real = job.real != 0;
     for (int i = threadIdx.x; i < N; i += G::NT) tw[i] = twn[i];
-    long sx, sy, sc;
-    plane_strides<N>(job.dim, sx, sy, sc);
+    const long sx = job.sx, sy = job.sy, sc = job.sc;
     const float inv = 1.0f / (float)(N * N);
     // one plane per CTA, or per cluster when the plane is split by rows
     sync_all<G>();  // (cluster) every CTA has started before any remote access
@@ -196,9 +220,8 @@ __global__ void __launch_bounds__(G::NT, 1) k_shear(ShearJobs jobs, const float2
             continue;
         }
         plane_load<G>(buf, p, sx, sy);
-        // per-plane phase factors (double): phase = 2 pi gc (cx gx(kx) + cy gy(ky)) / N;
-        // dim 1: a with n2 (x'), b with n3 (y'); 2: b with n1, a with n3; 3: a with n1, b with n2
-        const double cx = job.dim == 2 ? job.cb : job.ca, cy = job.dim == 2 ? job.ca : job.cb;
+        // per-plane phase factors (double): phase = 2 pi gc (cx gx(kx) + cy gy(ky)) / N
+        const double cx = job.cx, cy = job.cy;
         for (int L = threadIdx.x; L < N; L += G::NT) {
             const int k = G::scr(L);
             bool q;
@@ -259,12 +282,9 @@ __global__ void __launch_bounds__(G::NT, 1) k_shear1(ShearJobs jobs, const float
     float2 *f = tw + N, *h = f + N, *part = h + N;
     const ShearJob &job = jobs.j[blockIdx.y];
     const bool real = job.real != 0;
-    long sx, sy, sc;
-    plane_strides<N>(job.dim, sx, sy, sc);
-    // u: the axis of the one coefficient
-    const double cx = job.dim == 2 ? job.cb : job.ca, cy = job.dim == 2 ? job.ca : job.cb;
-    const long su = cy == 0.0 ? sx : sy, sw = cy == 0.0 ? sy : sx;
-    const double cu = cy == 0.0 ? cx : cy;
+    // x' is the axis of the one coefficient here
+    const long su = job.sx, sw = job.sy, sc = job.sc;
+    const double cu = job.cx;
     const float inv = 1.0f / (float)N;
     const int c = blockIdx.x, gc = [&] {
         bool q;
@@ -831,13 +851,35 @@ int rot_twiddles(int n, std::vector<float2> &h) {
 }
 
 namespace {
-Rows3 rows3_of(int n) { return Rows3{n, 256 / n}; }
-dim3 rows3_grid(const Rows3 &g, int jobs) { return dim3((g.n * g.n + g.rpb - 1) / g.rpb, jobs); }
+// the rotation without its empty shears
+struct Shear {
+    double ca, cb;
+    int dim;
+    bool real, none;
+};
+Shear shear_of(const RotPlan &pl, int k, int n) {
+    Shear h{no_shear(pl.a[k], n) ? 0.0 : pl.a[k], no_shear(pl.b[k], n) ? 0.0 : pl.b[k], pl.dim[k], k == 3, false};
+    h.none = h.ca == 0.0 && h.cb == 0.0;
+    return h;
+}
 
-// every shear of `count` rotations, each on its work volume, step by step:
-// the rotations' shears of one step share a launch (small volumes leave most of
-// the chip idle)
-int shear_all(const RotPlan *const *plans, int count, int n, float2 *S, const float2 *twn, int sms, cudaStream_t st) {
+// the fastest axis of the work volume: y or z when no shear of the rotation
+// runs along it, else x (256: x, its planes are split over a cluster)
+int fast_axis(const RotPlan &pl, int n) {
+    bool used[4] = {};
+    for (int k = 0; k < 4; ++k) {
+        const Shear h = shear_of(pl, k, n);
+        if (!h.none) used[h.dim] = true;
+    }
+    if (!pl.active || n == 256 || !used[1]) return 0;
+    return !used[2] ? 1 : !used[3] ? 2 : 0;
+}
+
+// every shear of `count` rotations, each on its work volume with fastest axis
+// f[j], step by step: the rotations' shears of one step share a launch (small
+// volumes leave most of the chip idle)
+int shear_all(const RotPlan *const *plans, const int *f, int count, int n, float2 *S, const float2 *twn, int sms,
+              cudaStream_t st) {
     const long stride = (long)n * n * n;
     int steps = 0;
     for (int j = 0; j < count; ++j)
@@ -849,12 +891,22 @@ int shear_all(const RotPlan *const *plans, int count, int n, float2 *S, const fl
             for (int j = 0; j < count; ++j) {
                 const RotPlan &pl = *plans[j];
                 if (!pl.active || s >= pl.num_step) continue;
-                ShearJob job{S + j * stride, no_shear(pl.a[k], n) ? 0.0 : pl.a[k], no_shear(pl.b[k], n) ? 0.0 : pl.b[k],
-                             pl.dim[k], k == 3};
-                const bool none = job.ca == 0.0 && job.cb == 0.0;
-                if (none && k < 3) continue;  // moves nothing
+                const Shear h = shear_of(pl, k, n);
+                if (h.none && !h.real) continue;  // moves nothing
+                int st3[3] = {1, n, n * n};
+                std::swap(st3[0], st3[f[j]]);
+                // the plane axes: dim 1: a with 2, b with 3; 2: a with 3, b with 1; 3: a with 1, b with 2
+                int ax = h.dim == 1 ? 1 : h.dim == 2 ? 2 : 0, bx = h.dim == 1 ? 2 : h.dim == 2 ? 0 : 1;
+                double ca = h.ca, cb = h.cb;
                 // (256: planes over a cluster, both kinds in k_shear)
-                if ((job.ca == 0.0 || job.cb == 0.0) && n != 256) one.j[n1++] = job;
+                const bool single = (ca == 0.0 || cb == 0.0) && n != 256;
+                // x' is the axis that moves, or of two the one of smaller stride
+                if (single ? ca == 0.0 && cb != 0.0 : st3[bx] < st3[ax]) {
+                    std::swap(ax, bx);
+                    std::swap(ca, cb);
+                }
+                const ShearJob job{S + j * stride, ca, cb, st3[ax], st3[bx], st3[h.dim - 1], h.real};
+                if (single) one.j[n1++] = job;
                 else two.j[n2++] = job;
             }
             int rc = n1 ? shear(n, one, n1, true, twn, sms, st) : 0;
@@ -863,6 +915,22 @@ int shear_all(const RotPlan *const *plans, int count, int n, float2 *S, const fl
         }
     return 0;
 }
+
+// the fastest axes of `count` work volumes; rotations that would take y and z
+// in one group all keep x (the copies of a group share one tile axis)
+void fast_axes(const RotPlan *const *plans, int count, int n, int *f) {
+    bool y = false, z = false;
+    for (int j = 0; j < count; ++j) {
+        f[j] = fast_axis(*plans[j], n);
+        y = y || f[j] == 1;
+        z = z || f[j] == 2;
+    }
+    if (y && z) std::fill(f, f + count, 0);
+    // a group with z-fastest volumes tiles over z; x-fastest ones follow
+    if (z)
+        for (int j = 0; j < count; ++j) f[j] = 2;
+}
+const dim3 kTileBlock(kTile, 8);
 }  // namespace
 
 // out = rotation of vol (both device [n][n][n] float, may alias), S = n^3 complex work
@@ -876,13 +944,14 @@ int rot_apply(const RotPlan &pl, int n, const float *vol, float *out, float2 *S,
         }
         return 0;
     }
-    const Rows3 g = rows3_of(n);
     const RotPlan *one = &pl;
-    k_rot_load<<<rows3_grid(g, 1), 256, 0, st>>>(vol, S, g, total);
+    RotPtrs j{};
+    fast_axes(&one, 1, n, j.f);
+    k_rot_load<false><<<tile_grid(n, 1), kTileBlock, 0, st>>>(vol, j, S, Axes{n}, total, n, 1);
     int rc = (int)cudaGetLastError();
-    if (!rc) rc = shear_all(&one, 1, n, S, twn, sms, st);
+    if (!rc) rc = shear_all(&one, j.f, 1, n, S, twn, sms, st);
     if (rc) return rc;
-    k_rot_store<<<rows3_grid(g, 1), 256, 0, st>>>(S, out, g);
+    k_rot_store<<<tile_grid(n, 1), kTileBlock, 0, st>>>(S, out, Axes{n}, j.f[0]);
     return (int)cudaGetLastError();
 }
 
@@ -890,16 +959,21 @@ int rot_apply(const RotPlan &pl, int n, const float *vol, float *out, float2 *S,
 // plan j, laterally centred in the window
 int rot_to_windows(const RotPlan *const *plans, int count, int n, const float *vol, float *const *V, int w, float2 *S,
                    const float2 *twn, int sms, cudaStream_t st) {
-    const Rows3 g = rows3_of(n);
     const long stride = (long)n * n * n;
-    RotPtrs out{};
-    for (int j = 0; j < count; ++j) out.p[j] = V[j];
-    k_rot_load<<<rows3_grid(g, count), 256, 0, st>>>(vol, S, g, stride);
+    RotPtrs j{};
+    for (int i = 0; i < count; ++i) {
+        j.p[i] = V[i];
+        if (w > n) {
+            const cudaError_t e = cudaMemsetAsync(V[i], 0, sizeof(float) * (size_t)n * w * w, st);
+            if (e != cudaSuccess) return (int)e;
+        }
+    }
+    fast_axes(plans, count, n, j.f);
+    k_rot_load<false><<<tile_grid(n, count), kTileBlock, 0, st>>>(vol, j, S, Axes{n}, stride, n, 1);
     int rc = (int)cudaGetLastError();
-    if (!rc) rc = shear_all(plans, count, n, S, twn, sms, st);
+    if (!rc) rc = shear_all(plans, j.f, count, n, S, twn, sms, st);
     if (rc) return rc;
-    const int rows = 256 / w;
-    k_rot_store_window<<<dim3((n * w + rows - 1) / rows, count), 256, 0, st>>>(S, out, g, stride, w);
+    k_rot_store_window<<<tile_grid(n, count), kTileBlock, 0, st>>>(S, j, Axes{n}, stride, w);
     return (int)cudaGetLastError();
 }
 
@@ -907,15 +981,15 @@ int rot_to_windows(const RotPlan *const *plans, int count, int n, const float *v
 // gradient G_j (FP64 [ns][w][w], each slab on its b voxels)
 int rot_accumulate(const RotPlan *const *plans, int count, int n, const double *const *G, int w, int b, double *acc,
                    bool zero, float2 *S, const float2 *twn, int sms, cudaStream_t st) {
-    const Rows3 g = rows3_of(n);
     const long stride = (long)n * n * n;
-    RotPtrs in{};
-    for (int j = 0; j < count; ++j) in.p[j] = const_cast<double *>(G[j]);
-    k_rot_load_slabs<<<rows3_grid(g, count), 256, 0, st>>>(in, S, g, stride, w, b);
+    RotPtrs j{};
+    for (int i = 0; i < count; ++i) j.p[i] = const_cast<double *>(G[i]);
+    fast_axes(plans, count, n, j.f);
+    k_rot_load<true><<<tile_grid(n, count), kTileBlock, 0, st>>>(nullptr, j, S, Axes{n}, stride, w, b);
     int rc = (int)cudaGetLastError();
-    if (!rc) rc = shear_all(plans, count, n, S, twn, sms, st);
+    if (!rc) rc = shear_all(plans, j.f, count, n, S, twn, sms, st);
     if (rc) return rc;
-    k_rot_accumulate<<<rows3_grid(g, 1), 256, 0, st>>>(S, acc, g, stride, count, zero ? 1 : 0);
+    k_rot_accumulate<<<tile_grid(n, 1), kTileBlock, 0, st>>>(S, acc, j, Axes{n}, stride, count, zero ? 1 : 0);
     return (int)cudaGetLastError();
 }
 
