@@ -144,28 +144,12 @@ struct ShearJobs {
 };
 
 // A plane between global memory (rows at stride sw, elements at su) and shared
-// memory; the loads are asynchronous (plane_wait).  Lanes run along the
-// contiguous axis: along u, or 4 rows by 8 elements, which covers 32-byte
-// sectors with two-way bank conflicts.
-template <class G>
-__device__ __forceinline__ void plane_pos(int i, bool across, int &r, int &u) {
-    constexpr int N = G::N;
-    if (across) {
-        const int q = i / (4 * N), m = i % (4 * N);
-        r = 4 * q + m % 4;
-        u = m / 4;
-    } else {
-        r = i / N;
-        u = i % N;
-    }
-}
+// memory, lanes along the rows; the loads are asynchronous (plane_wait)
 template <class G>
 __device__ __forceinline__ void plane_load(float2 *buf, const float2 *p, long su, long sw) {
     const int yb = G::ybase();
-    const bool across = sw == 1 && G::CL == 1;
     for (int i = threadIdx.x; i < G::ROWS * G::N; i += G::NT) {
-        int r, u;
-        plane_pos<G>(i, across, r, u);
+        const int r = i / G::N, u = i % G::N;
         const uint32_t d = (uint32_t)__cvta_generic_to_shared(buf + G::at(r, u));
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(p + (long)G::gy(yb, r) * sw + (long)u * su)
                      : "memory");
@@ -176,10 +160,8 @@ __device__ __forceinline__ void plane_wait() { asm volatile("cp.async.wait_group
 template <class G>
 __device__ __forceinline__ void plane_store(const float2 *buf, float2 *p, long su, long sw, bool real) {
     const int yb = G::ybase();
-    const bool across = sw == 1 && G::CL == 1;
     for (int i = threadIdx.x; i < G::ROWS * G::N; i += G::NT) {
-        int r, u;
-        plane_pos<G>(i, across, r, u);
+        const int r = i / G::N, u = i % G::N;
         float2 v = buf[G::at(r, u)];
         if (real) v.y = 0.f;
         p[(long)G::gy(yb, r) * sw + (long)u * su] = v;
@@ -264,100 +246,98 @@ __global__ void __launch_bounds__(G::NT, 1) k_shear(ShearJobs jobs, const float2
 }
 
 // A shear with one coefficient (a rotation about a volume axis has only such
-// ones): the plane's rows along the other axis u move on their own, except that
-// the spectrum's Nyquist line across the rows stays (its grid is zeroed), so
+// ones): the plane's lines along that axis u move on their own, except that the
+// spectrum's Nyquist line across them (along the other axis w) stays, its grid
+// being zeroed, so
 //   out(k, w) = e(k) S(k, w) + (1 - e(k)) (-1)^w c(k),
 //   c(k) = sum_w (-1)^w S(k, w) / N
 // with e the phase along u: one transform along u each way and one alternating
-// column sum, 4 passes over the plane instead of 7.
-template <class G>
-constexpr int kSumParts = G::NT / G::N > 4 ? 4 : G::NT / G::N;
+// row sum.  w is the plane's contiguous axis (the work volume's fastest one),
+// so u runs down the columns: three column passes, with the phase between two
+// transforms in the middle one (mid reconstruction, two iterations: 32.7 ms with
+// u along the rows and the plane transposed in shared memory, 31.1 this way).  The row sums sit in the rows' last pad cells
+// and go through the forward transform as one more column.
 template <class G>
 __global__ void __launch_bounds__(G::NT, 1) k_shear1(ShearJobs jobs, const float2 *twn) {
-    constexpr int N = G::N, R1 = G::R1, R2 = G::R2, PARTS = kSumParts<G>;
-    static_assert(PARTS >= 1, "a thread per column");
+    constexpr int N = G::N, R1 = G::R1, R2 = G::R2, S = G::S;
+    static_assert(S > N, "a pad cell at the end of every row");
+    using O = Own<G>;
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm;
     float2 *tw = buf + G::FIELD;
-    float2 *f = tw + N, *h = f + N, *part = h + N;
+    float2 *f = tw + N, *h = f + N;
     const ShearJob &job = jobs.j[blockIdx.y];
     const bool real = job.real != 0;
-    // x' is the axis of the one coefficient here
-    const long su = job.sx, sw = job.sy, sc = job.sc;
-    const double cu = job.cx;
     const float inv = 1.0f / (float)N;
-    const int c = blockIdx.x, gc = [&] {
-        bool q;
-        return rot_grid_val(c, N, &q);
-    }();
-    float2 *p = job.S + (long)c * sc;
-    if (gc == 0 || cu == 0.0) {
-        plane_keep<G>(p, su, sw, real);
+    const int c = blockIdx.x;
+    bool qc;
+    const int gc = rot_grid_val(c, N, &qc);
+    float2 *p = job.S + (long)c * job.sc;
+    if (gc == 0 || job.cy == 0.0) {
+        plane_keep<G>(p, job.sx, job.sy, real);
         return;
     }
-    plane_load<G>(buf, p, su, sw);
+    plane_load<G>(buf, p, job.sx, job.sy);
     for (int L = threadIdx.x; L < N; L += G::NT) {
         tw[L] = twn[L];
         bool q;
         const int g = rot_grid_val(G::scr(L), N, &q);
         double s, co;
-        sincospi(2.0 * (double)gc * cu * (double)g / (double)N, &s, &co);  // the Nyquist grid value is 0
-        f[L] = make_float2((float)co, (float)s);
+        sincospi(2.0 * (double)gc * job.cy * (double)g / (double)N, &s, &co);  // the Nyquist grid value is 0
+        f[L] = make_float2((float)co * inv, (float)s * inv);
     }
     plane_wait();
     __syncthreads();
-    row_passA<G, 0, -1>(buf, tw, NoOp{});
-    sync_rows();
-    row_passB<G, -1>(buf);
-    __syncthreads();
-    if (threadIdx.x < PARTS * N) {
-        const int L = threadIdx.x % N, w0 = threadIdx.x / N;
+    // alternating row sums: w and w + 32 have one sign
+    for (int r = O::warp() * O::RPW; r < (O::warp() + 1) * O::RPW; ++r) {
         float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 4
-        for (int w = w0; w < N; w += PARTS) {
-            const float2 v = buf[G::at(w, L)];
-            acc = (w & 1) ? csub(acc, v) : cadd(acc, v);
-        }
-        part[w0 * N + L] = acc;
-    }
-    __syncthreads();
-    for (int L = threadIdx.x; L < N; L += G::NT) {
-        float2 acc = part[L];
+        for (int w = O::lane(); w < N; w += 32) acc = cadd(acc, buf[G::at(r, w)]);
+        if (O::lane() & 1) acc = make_float2(-acc.x, -acc.y);
 #pragma unroll
-        for (int q = 1; q < PARTS; ++q) acc = cadd(acc, part[q * N + L]);
-        const float2 e = f[L];
-        h[L] = cscale(cmul(make_float2(1.f - e.x, -e.y), acc), inv * inv);
-        f[L] = cscale(e, inv);
+        for (int o = 16; o > 0; o >>= 1) {
+            acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+            acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+        }
+        if (O::lane() == 0) buf[r * S + S - 1] = acc;
     }
     __syncthreads();
-    // inverse row pass B with the phase
-    using O = Own<G>;
-    const int y0 = O::warp() * O::RPW;
-#pragma unroll 1
-    for (int tau = O::lane(); tau < O::RPW * R2; tau += 32) {
-        const int k2 = tau % R2, y = y0 + tau / R2;
-        float2 *b = buf + y * G::S + G::xb0(k2);
-        float2 v[R1];
+    if (O::warp() == 0) {
+        // the sums' column, and its share of every element of a row of the spectrum
+        float2 *b = buf + S - 1;
+        if (O::lane() < R1) {
+            float2 v[R2];
+#pragma unroll
+            for (int j = 0; j < R2; ++j) v[j] = b[(O::lane() + R1 * j) * S];
+            DFT<R2, -1>::run(v);
+#pragma unroll
+            for (int j = 0; j < R2; ++j) b[(O::lane() + R1 * j) * S] = j ? cmul(v[j], twN<G, -1>(tw, O::lane(), j)) : v[j];
+        }
+        __syncwarp();
+        if (O::lane() < R2) {
+            float2 v[R1];
+#pragma unroll
+            for (int j = 0; j < R1; ++j) v[j] = b[(j + R1 * O::lane()) * S];
+            DFT<R1, -1>::run(v);
+#pragma unroll
+            for (int j = 0; j < R1; ++j) {
+                const float2 e = f[j + R1 * O::lane()];
+                h[j + R1 * O::lane()] = cscale(cmul(make_float2(inv - e.x, -e.y), v[j]), inv);
+            }
+        }
+    }
+    col_passA<G, -1, true>(buf, tw);
+    __syncthreads();
+    col_passB<G, -1, +1>(buf, [&](int y0, int x, float2 *v) {
 #pragma unroll
         for (int j = 0; j < R1; ++j) {
-            const float2 t = cmul(b[G::xb(k2, j)], f[R1 * k2 + j]), n = h[R1 * k2 + j];
-            v[j] = (y & 1) ? csub(t, n) : cadd(t, n);
+            const float2 t = cmul(v[j], f[y0 + j]);
+            v[j] = (x & 1) ? csub(t, h[y0 + j]) : cadd(t, h[y0 + j]);
         }
-        DFT<R1, +1>::run(v);
-#pragma unroll
-        for (int j = 0; j < R1; ++j) b[G::xb(k2, j)] = v[j];
-    }
-    sync_rows();
-    const bool direct = su == 1;  // rows contiguous in memory: straight from pass A
-    row_passA<G, +1, 0>(buf, tw, [&](int y, int n1, float2 *v) {
-        if (direct)
-#pragma unroll
-            for (int j = 0; j < R2; ++j)
-                p[(long)y * sw + n1 + R1 * j] = make_float2(v[j].x, real ? 0.f : v[j].y);
     });
-    if (direct) return;
+    sync_cols<G>();
+    col_passA<G, +1, false>(buf, tw);
     __syncthreads();
-    plane_store<G>(buf, p, su, sw, real);
+    plane_store<G>(buf, p, job.sx, job.sy, real);
 }
 
 template <class G>
@@ -382,7 +362,7 @@ static int launch_shear(const ShearJobs &jobs, int count, bool one, const float2
         return (int)cudaLaunchKernelEx(&cfg, k, jobs, twn);
     } else {
         auto k = one ? k_shear1<G> : k_shear<G>;
-        const size_t smem = sizeof(float2) * ((size_t)G::FIELD + (one ? 3 + kSumParts<G> : 3) * G::N);
+        const size_t smem = sizeof(float2) * ((size_t)G::FIELD + 3 * G::N);
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         // planes in flight: one per CTA (k_shear1: one plane per CTA in all)
@@ -900,8 +880,8 @@ int shear_all(const RotPlan *const *plans, const int *f, int count, int n, float
                 double ca = h.ca, cb = h.cb;
                 // (256: planes over a cluster, both kinds in k_shear)
                 const bool single = (ca == 0.0 || cb == 0.0) && n != 256;
-                // x' is the axis that moves, or of two the one of smaller stride
-                if (single ? ca == 0.0 && cb != 0.0 : st3[bx] < st3[ax]) {
+                // y' is the axis of a single coefficient; x' of two the one of smaller stride
+                if (single ? ca != 0.0 : st3[bx] < st3[ax]) {
                     std::swap(ax, bx);
                     std::swap(ca, cb);
                 }
