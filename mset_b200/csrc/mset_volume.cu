@@ -148,9 +148,17 @@ __device__ __forceinline__ void tv_project(float q1, float q2, float q3, float &
 // field is read from src and written to dst, so the neighbours' old values
 // survive.  Per voxel it moves 16 B of source and input (and 1 / zc + 1 / ty
 // of them again), 12 of P and 24 of results, against 20 + 52 in two kernels
-// with D in memory, and half the launches: 164.8 -> 113.4 us per FISTA iteration
-// at 256 x 256 x 192 (6.0 TB/s of HBM), 24.8 -> 20.6 at 128^3 (L2 and the
-// chain of a step), 16.3 -> 10.3 at 96^3.
+// with D in memory, and half the launches: 164.8 -> 110.3 us per FISTA iteration
+// at 256 x 256 x 192 (6.0 TB/s of HBM), 24.8 -> 20.5 at 128^3 (L2 and the
+// chain of a step), 16.3 -> 10.0 at 96^3, 12.3 -> 6.1 at 64^3.
+//
+// Each iteration's kernel is set up while the one before drains (programmatic
+// dependent launch; the wait stands before the first access): 108.2, 18.6, 8.8
+// and 3.9 us there, 3.4 against 6.1 at 48^3; inside a captured iteration, whose
+// launches cost less, 2.5% of it at 48^3 and 0.5 to 2% above.  The kernels do not
+// signal early: CTAs of the next iteration then take places among the running
+// ones, whose neighbours share slices in L2 (129.7 us at 256 x 256 x 192, 19.8 at
+// 128^3).
 struct Quad {
     float v[4];
 };
@@ -186,6 +194,8 @@ __global__ void __launch_bounds__(256) k_tv_march(const float *src, float *dst, 
     const int y0 = (blockIdx.x % tiles) * ty, z0 = (blockIdx.x / tiles) * zc, z1 = min(z0 + zc, g.n3);
     const int rows = min(ty, g.n2 - y0);
     const bool on = r < rows, halo = r == 0;
+    // the iteration before has finished and its stores are visible
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int y = y0 + (on ? r : 0), ym = y == 0 ? g.n2 - 1 : y - 1;
     const int yh = y0 + rows == g.n2 ? 0 : y0 + rows, yhm = y0 + rows - 1;
     float *cur = dsm, *nxt = dsm + (ty + 1) * g.n1;
@@ -555,8 +565,21 @@ int tv_prox(const TvArgs &a, cudaStream_t st) {
             t = (1.0 + std::sqrt(1.0 + 4.0 * t0 * t0)) / 2.0;  // TV_FISTA_method.m:31
             const double m = (t0 - 1.0) / t;
             if (march) {
-                if (a.fista) k_tv_march<true><<<grid, q1 * ty, sm, st>>>(src, dst, a.P, a.in, rows, ty, zc, inv_lam, tau, m);
-                else k_tv_march<false><<<grid, q1 * ty, sm, st>>>(src, dst, nullptr, a.in, rows, ty, zc, inv_lam, tau, m);
+                // set up while the iteration before drains; the first follows
+                // the clearing of its fields
+                cudaLaunchAttribute chain = {};
+                chain.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                chain.val.programmaticStreamSerializationAllowed = 1;
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3(grid);
+                cfg.blockDim = dim3(q1 * ty);
+                cfg.dynamicSmemBytes = sm;
+                cfg.stream = st;
+                cfg.attrs = &chain;
+                cfg.numAttrs = it > 0 ? 1 : 0;
+                e = cudaLaunchKernelEx(&cfg, a.fista ? k_tv_march<true> : k_tv_march<false>, (const float *)src, dst,
+                                       a.fista ? a.P : nullptr, a.in, rows, ty, zc, inv_lam, tau, m);
+                if (e != cudaSuccess) return (int)e;
                 std::swap(src, dst);
             } else {
                 k_tv_d<<<g, bt, 0, st>>>(a.fista ? a.Y : a.P, a.in, a.D, rows, inv_lam);
