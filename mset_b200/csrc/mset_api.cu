@@ -747,7 +747,9 @@ int mset_forward_position(mset_session *s, int mode, int k, float row, float col
     if (psi0_out) CK(cudaMemcpyAsync(psi0_out, s->save.p, sizeof(float2) * n2, cudaMemcpyDeviceToHost, s->st));
     double e = 0;
     CK(cudaMemcpyAsync(&e, s->step_err.p, sizeof(double), cudaMemcpyDeviceToHost, s->st));
-    CK(cudaStreamSynchronize(s->st));
+    // (waits for the stream; a failed forward leaves no step for an adjoint)
+    rc = take_fault(s);
+    if (rc) return rc;
     if (resi_out) {
         float2 *ro = reinterpret_cast<float2 *>(resi_out);
         for (int Ly = 0; Ly < n; ++Ly) {
