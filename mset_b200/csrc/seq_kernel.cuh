@@ -43,6 +43,7 @@
 // mset_dispatch.cu.
 #pragma once
 #include "mset_kernels_impl.cuh"
+#include "seq_exchange.h"
 
 namespace mset {
 
@@ -116,8 +117,7 @@ struct SeqKernel {
     uint32_t peer_bars[CL];
     uint32_t row_base = 0, row_bar = 0;  // the CTA that owns the rows of the column pass-A task
     int rank;
-    unsigned phr = 0, phc = 0;  // completed phases of the row and column exchanges
-    bool dead = false;          // a wait gave up: no further waits
+    SeqProgress at_x;  // exchanges so far
     // pass-A tasks: row (yr, n1r) and column (xc, n1c); pass-B task (lb, kb) of
     // rows and of columns alike
     int n1r, lr, n1c, lc, lb, kb;
@@ -207,20 +207,24 @@ struct SeqKernel {
         if constexpr (CL == 1) {
             __syncthreads();
         } else {
-            unsigned &ph = which ? phc : phr;
-            if (!dead && !mbar_wait_cluster(bars + 8u * which, ph & 1u)) {
-                if (a.fault) atomicOr(a.fault, 1u);
-                mbar_wait_cluster(bars + 8u * which, ph & 1u);  // let late pushes land
-                dead = true;
+            bool done = true;
+            if (at_x.waits()) {
+                const unsigned par = at_x.parity(which);
+                done = mbar_wait_cluster(bars + 8u * which, par);
+                if (!done) {
+                    if (a.fault) atomicOr(a.fault, 1u);
+                    mbar_wait_cluster(bars + 8u * which, par);  // let late pushes land
+                }
             }
-            ++ph;
-            if (!dead) arm(which);
+            at_x.waited(which, done);
+            if (at_x.arms()) arm(which);
         }
     }
     // this CTA's element `off` of the row (which = 0) or column buffer of CTA q
     __device__ __forceinline__ void push(int which, uint32_t base, uint32_t bar, int off, float2 v) const {
         if constexpr (CL == 1) (which ? colbuf : rowbuf)[off] = v;
-        else st_async(base + (uint32_t)sizeof(float2) * (uint32_t)((which ? G::COL : 0) + off), v, bar + 8u * which);
+        else if (at_x.sends())
+            st_async(base + (uint32_t)sizeof(float2) * (uint32_t)((which ? G::COL : 0) + off), v, bar + 8u * which);
     }
 
     static __device__ __forceinline__ void load_a(const float2 *p, float2 *v) {
