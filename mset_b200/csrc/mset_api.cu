@@ -462,9 +462,9 @@ int launch_sequential(mset_session *s, bool cluster, int method, int adjoint, in
     return 0;
 }
 
-// The position kernel waits, with a bound, for the bulk copies that stage
-// its operands in shared memory; a wait that gave up sets the session's
-// fault word.  Read (and clear) it where a call hands results back.
+// The position kernels wait, with a bound, for the bulk copies that stage their
+// operands in shared memory and for the pushes of their cluster's other CTAs
+// (seq_kernel.cuh); a wait that gave up sets the session's fault word.  Read (and clear) it where a call hands results back.
 int take_fault(mset_session *s) {
     if (!s->fault.p) return 0;
     unsigned f = 0;
@@ -473,8 +473,9 @@ int take_fault(mset_session *s) {
     if (!f) return 0;
     CK(cudaMemsetAsync(s->fault.p, 0, sizeof(unsigned), s->st));
     CK(cudaStreamSynchronize(s->st));
-    return fail(MSET_E_CUDA, "a bulk copy into shared memory did not complete within the position kernel's "
-                             "bounded wait; the results of this call are invalid");
+    return fail(MSET_E_CUDA, "a bounded wait of the position kernel gave up (for a bulk copy into shared memory, or "
+                             "for the rows or columns that other CTAs of its cluster send); the results of this "
+                             "call are invalid");
 }
 
 int effective_mode(const mset_session *s, int method, int mode) {

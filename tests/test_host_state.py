@@ -15,3 +15,13 @@ report(forward=outcome(s.step02, 0, 32.0, 32.0), adjoint=outcome(s.step03), word
     assert r["forward"][0] == MSET_E_CUDA
     assert r["adjoint"][0] == MSET_E_STATE  # no forward to go back from
     assert r["word"] == 0 and r["again"] == 0 and r["then"] == 0
+
+
+def test_the_error_of_a_wait_names_what_may_have_been_waited_for():
+    r = hostcuda.run("""
+s = sequential(64)
+(C.c_uint * 1).from_address(F.fake_alloc(0))[0] = 1
+report(run=outcome(s.run, 1))
+""")
+    assert r["run"][0] == MSET_E_CUDA
+    assert "bulk copy" in r["run"][1] and "cluster" in r["run"][1]
