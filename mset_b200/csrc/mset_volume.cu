@@ -9,8 +9,9 @@
 // HBM/L2-bound elementwise work: grid-stride loops over 148 x 8 CTAs (the
 // scalar TV stencils: over rows, one CTA per row).  TV runs on one of three
 // routes (tv_prox): every iteration in one cluster launch where the volume fits
-// its shared memory, one marching kernel per iteration where rows are whole
-// float4 groups, else two kernels per iteration.
+// its shared memory and few slices fall to a CTA (tv_cluster_pays), one marching
+// kernel per iteration where rows are whole float4 groups, else two kernels per
+// iteration.
 #include <algorithm>
 #include <cmath>
 
@@ -267,7 +268,8 @@ __global__ void __launch_bounds__(256) k_tv_march(const float *src, float *dst, 
 // bound the kernels above at these sizes; here it is the arithmetic of one
 // CTA's slices (square root, three divisions, FP64 momentum per voxel), so the
 // cluster is the largest one (24^3: 8.1 us per iteration of two launches, 2.5 on
-// 8 CTAs, 1.9 on 16; 32^3: 8.2, 6.6, 4.1).  Per iteration a CTA
+// 8 CTAs, 1.9 on 16) and its route ends where a CTA's share gets long
+// (tv_cluster_pays).  Per iteration a CTA
 // computes D of its slices and of the one above them, steps, and hands its
 // bottom slice's new dual values to the CTA below and its top slice's third
 // component to the CTA above (two halo buffers in turn, so one cluster barrier
@@ -468,19 +470,42 @@ __global__ void k_update(float *rec, const double *acc, long n, float step0) {
 }  // namespace
 
 namespace {
+// rows of whole float4 groups, at most one CTA long
+inline bool tv_rows4(int n1) { return n1 % 4 == 0 && n1 <= 1024; }
+
+// Whether K slices per CTA of planes of A voxels run on the cluster kernel; march:
+// the marching kernel is the other choice, else two kernels per iteration are.
+// The cluster's time per iteration is a thread's chain through its columns, 0.3 to
+// 0.6 us a slice by the warps there are, on top of 0.9; the march takes 2.4 to 3.0
+// whatever the volume up to 40^3.  Microseconds per iteration in a captured
+// graph (one B200, cluster / march; bare launches of the march cost 0.2 more):
+//   FISTA  24^3 (K 2)  1.87 / 2.66   16x16x64 (K 4)  2.28 / 2.49   24x24x48 (K 3)  2.50 / 2.68
+//          24x24x64 (K 4)  3.08 / 2.66   24x32x48 (K 3)  2.84 / 2.67   16x16x128 (K 8)  3.95 / 2.46
+//          32^3 (K 2, two columns a thread)  4.16 / 2.70   24x24x160 (K 10)  6.42 / 3.25
+//   TV     24x24x48 (K 3)  1.84 / 2.45   24x24x64 (K 4)  2.23 / 2.44   24x24x96 (K 6)  2.98 / 2.60
+//          16x16x128 (K 8)  2.71 / 2.28   32^3 (K 2)  3.28 / 2.47
+// Against two kernels per iteration (8.2 bare for FISTA and TV alike):
+//   FISTA  30x30x60 (K 4)  4.3   34^3 (K 3, two columns)  5.6   26x26x100 (K 7)  5.3
+//          9x9x200 (K 13)  5.6   6x6x500 (K 32)  13.0   5x5x4000 (K 250)  97.9 (two kernels: 18.4)
+inline bool tv_cluster_pays(long A, int K, bool fista, bool march) {
+    const long columns = (A + 991) / 992;  // per thread
+    if (march) return columns == 1 && K <= 4 && A * K <= (fista ? 1728 : 2304);
+    return columns * K <= 16;
+}
+
 // launch configuration of the cluster kernel over a volume; false: it does not
-// fit one cluster's shared memory
+// fit one cluster's shared memory, or another route is faster
 template <bool FISTA>
 struct TvCluster {
     cudaLaunchAttribute at[1] = {};
     cudaLaunchConfig_t cfg = {};
     int K = 0;
-    bool prepare(int n1, int n2, int n3, cudaStream_t st) {
+    bool prepare(int n1, int n2, int n3, bool march, cudaStream_t st) {
         const long A = (long)n1 * n2;
         for (int cl : {kTvCl, 8}) {
             K = (n3 + cl - 1) / cl;
             const long bytes = tv_cluster_floats(A, K, FISTA) * (long)sizeof(float);
-            if (bytes > 220 * 1024) continue;
+            if (bytes > 220 * 1024 || !tv_cluster_pays(A, K, FISTA, march)) continue;
             auto k = k_tv_cluster<FISTA>;
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
                 (cl > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
@@ -501,18 +526,18 @@ struct TvCluster {
         return false;
     }
 };
-// every iteration in one launch; -1: the volume does not fit
+// every iteration in one launch; -1: not on this route
 template <bool FISTA>
-int tv_cluster(const TvArgs &a, const Rows &rows, float inv_lam, float tau, cudaStream_t st) {
+int tv_cluster(const TvArgs &a, bool march, const Rows &rows, float inv_lam, float tau, cudaStream_t st) {
     TvCluster<FISTA> c;
-    if (!c.prepare(a.n1, a.n2, a.n3, st)) return -1;
+    if (!c.prepare(a.n1, a.n2, a.n3, march, st)) return -1;
     return (int)cudaLaunchKernelEx(&c.cfg, k_tv_cluster<FISTA>, a.P, a.in, rows, c.K, inv_lam, tau, a.niter);
 }
 }  // namespace
 
 bool tv_wants_second(int n1, int n2, int n3, bool fista) {
     TvCluster<true> c;
-    return fista && n1 % 4 == 0 && n1 <= 1024 && !c.prepare(n1, n2, n3, nullptr);
+    return fista && tv_rows4(n1) && !c.prepare(n1, n2, n3, true, nullptr);
 }
 
 int tv_prox(const TvArgs &a, cudaStream_t st) {
@@ -532,14 +557,16 @@ int tv_prox(const TvArgs &a, cudaStream_t st) {
     float *res = a.P;  // the dual field after the last iteration
     cudaError_t e;
     int rc = -1;
-    if (a.niter > 0) rc = a.fista ? tv_cluster<true>(a, rows, inv_lam, tau, st) : tv_cluster<false>(a, rows, inv_lam, tau, st);
+    // one kernel per iteration needs a second dual field: Y2 (FISTA), or P and Y
+    // in turn
+    const bool march = tv_rows4(a.n1) && (!a.fista || a.Y2);
+    if (a.niter > 0)
+        rc = a.fista ? tv_cluster<true>(a, march, rows, inv_lam, tau, st)
+                     : tv_cluster<false>(a, march, rows, inv_lam, tau, st);
     if (rc > 0) return rc;
     if (rc < 0) {
         if ((e = cudaMemsetAsync(a.P, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
         if ((e = cudaMemsetAsync(a.Y, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
-        // one kernel per iteration needs a second dual field: Y2 (FISTA), or P
-        // and Y in turn
-        const bool march = vec && a.n1 <= 1024 && (!a.fista || a.Y2);
         const int q1 = std::max(1, a.n1 / 4), ty = std::max(1, std::min(128 / q1, a.n2));
         const int tiles = (a.n2 + ty - 1) / ty;
         int zc = 1;

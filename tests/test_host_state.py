@@ -25,3 +25,38 @@ report(run=outcome(s.run, 1))
 """)
     assert r["run"][0] == MSET_E_CUDA
     assert "bulk copy" in r["run"][1] and "cluster" in r["run"][1]
+
+
+# (n3, n2, n1), FISTA, kernel of an iteration, launches of it in 5 iterations: few
+# slices per CTA and a column per thread run in one cluster launch, more on the
+# marching kernel, rows of other lengths in the cluster up to 16 columns of
+# slices per thread, else on two kernels
+TV_ROUTES = [
+    ((24, 24, 24), True, "k_tv_cluster", 1), ((48, 24, 24), True, "k_tv_cluster", 1),
+    ((64, 24, 24), True, "k_tv_march", 5), ((64, 24, 24), False, "k_tv_cluster", 1),
+    ((96, 24, 24), True, "k_tv_march", 5), ((96, 24, 24), False, "k_tv_march", 5),
+    ((64, 16, 16), True, "k_tv_cluster", 1), ((128, 16, 16), True, "k_tv_march", 5),
+    ((32, 32, 32), True, "k_tv_march", 5), ((32, 32, 32), False, "k_tv_march", 5),
+    ((8, 48, 48), True, "k_tv_march", 5), ((6000, 4, 4), True, "k_tv_march", 5),
+    ((128, 128, 128), True, "k_tv_march", 5),
+    ((30, 30, 30), True, "k_tv_cluster", 1), ((34, 34, 34), True, "k_tv_cluster", 1),
+    ((200, 9, 9), True, "k_tv_cluster", 1), ((500, 6, 6), True, "k_tv_step", 5),
+    ((4000, 5, 5), False, "k_tv_step", 5), ((60, 50, 50), True, "k_tv_step", 5),
+]
+
+
+def test_tv_runs_on_the_route_that_measured_fastest():
+    r = hostcuda.run("""
+got = []
+with Session() as s:
+    for shape, fista in %r:
+        F.fake_clear_log()
+        s.tv(np.zeros(shape, np.float32), 0.1, 5, fista)
+        got.append(launched())
+report(got=got, bad=F.fake_bad())
+""" % [(shape, fista) for shape, fista, _, _ in TV_ROUTES])
+    assert r["bad"] == 0
+    for (shape, fista, kernel, launches), names in zip(TV_ROUTES, r["got"]):
+        assert sum(kernel in x for x in names) == launches, (shape, fista, names)
+        per_iteration = ("k_tv_cluster", "k_tv_march", "k_tv_step")
+        assert sum(any(k in x for k in per_iteration) for x in names) == launches, (shape, fista, names)
