@@ -72,7 +72,7 @@ inline dim3 tile_grid(int n, int jobs) {
     const int nt = (n + kTile - 1) / kTile;
     return dim3(nt * nt * n, jobs);
 }
-__device__ __forceinline__ int tile_axis(int f) { return f == 2 ? 2 : 1; }
+__host__ __device__ __forceinline__ int tile_axis(int f) { return f == 2 ? 2 : 1; }
 
 // S_j = ifftshift of vol (grads null), or of a tilt's slab gradient (FP64
 // [ns][w][w]), each slab on its b voxels, cropped to the volume
@@ -111,12 +111,11 @@ __global__ void __launch_bounds__(256) k_rot_store_window(const float2 *S, RotPt
     for_tile(x.n, g, true, tile,
              [&](int i1, int i2, int i3, float &t) { V[((long)i3 * w + i2 + o) * w + i1 + o] = t; });
 }
-// acc (+)= sum over the jobs, in their order, of fftshift(real(S_j)), FP64
+// acc (+)= sum over the jobs, in their order, of fftshift(real(S_j)), FP64; g: the
+// jobs' common tile axis (every job's tile is the same voxels)
 __global__ void __launch_bounds__(256) k_rot_accumulate(const float2 *S, double *acc, RotPtrs j, Axes x, long stride,
-                                                        int jobs, int zero) {
+                                                        int jobs, int g, int zero) {
     __shared__ float tile[kTile][kTile + 1];
-    // every job's tile is the same voxels: they share one tile axis (shear_all)
-    const int g = tile_axis(j.f[0]);
     for (int k = 0; k < jobs; ++k) {
         const int f = j.f[k];
         __syncthreads();
@@ -896,19 +895,9 @@ int shear_all(const RotPlan *const *plans, const int *f, int count, int n, float
     return 0;
 }
 
-// the fastest axes of `count` work volumes; rotations that would take y and z
-// in one group all keep x (the copies of a group share one tile axis)
+// each work volume keeps its own rotation's fastest axis
 void fast_axes(const RotPlan *const *plans, int count, int n, int *f) {
-    bool y = false, z = false;
-    for (int j = 0; j < count; ++j) {
-        f[j] = fast_axis(*plans[j], n);
-        y = y || f[j] == 1;
-        z = z || f[j] == 2;
-    }
-    if (y && z) std::fill(f, f + count, 0);
-    // a group with z-fastest volumes tiles over z; x-fastest ones follow
-    if (z)
-        for (int j = 0; j < count; ++j) f[j] = 2;
+    for (int j = 0; j < count; ++j) f[j] = fast_axis(*plans[j], n);
 }
 const dim3 kTileBlock(kTile, 8);
 }  // namespace
@@ -969,8 +958,24 @@ int rot_accumulate(const RotPlan *const *plans, int count, int n, const double *
     int rc = (int)cudaGetLastError();
     if (!rc) rc = shear_all(plans, j.f, count, n, S, twn, sms, st);
     if (rc) return rc;
-    k_rot_accumulate<<<tile_grid(n, 1), kTileBlock, 0, st>>>(S, acc, j, Axes{n}, stride, count, zero ? 1 : 0);
-    return (int)cudaGetLastError();
+    // y-fastest and z-fastest volumes tile over different axes: one launch per run
+    // of neighbours that share one (x-fastest volumes go with either), in order
+    for (int i0 = 0; i0 < count;) {
+        RotPtrs part{};
+        int g = 0, m = 0;
+        for (; i0 + m < count; ++m) {
+            const int f = j.f[i0 + m];
+            if (f && g && f != g) break;
+            if (f) g = f;
+            part.f[m] = f;
+        }
+        k_rot_accumulate<<<tile_grid(n, 1), kTileBlock, 0, st>>>(S + i0 * stride, acc, part, Axes{n}, stride, m,
+                                                                 tile_axis(g), zero && i0 == 0 ? 1 : 0);
+        rc = (int)cudaGetLastError();
+        if (rc) return rc;
+        i0 += m;
+    }
+    return 0;
 }
 
 }  // namespace mset

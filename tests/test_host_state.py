@@ -60,3 +60,34 @@ report(got=got, bad=F.fake_bad())
         assert sum(kernel in x for x in names) == launches, (shape, fista, names)
         per_iteration = ("k_tv_cluster", "k_tv_march", "k_tv_step")
         assert sum(any(k in x for k in per_iteration) for x in names) == launches, (shape, fista, names)
+
+
+def test_rotations_of_a_group_never_shear_along_the_contiguous_axis():
+    """a rotation about a volume axis leaves one axis unsheared, x among the
+    rows or the work volume's own fastest one: whatever else is in its group, its
+    shears run along strided axes (planes that hold the contiguous one)"""
+    r = hostcuda.run("""
+class Job(C.Structure):  # ShearJob of csrc/mset_rotate.cu
+    _fields_ = [("S", C.c_void_p), ("cx", C.c_double), ("cy", C.c_double), ("sx", C.c_int), ("sy", C.c_int),
+                ("sc", C.c_int), ("real", C.c_int)]
+n, turns = 24, [(0, 1), (1, 0), (2, 1), (0, 2), (1, 2)]  # (angle that is not zero, its sign or size)
+b = batched(32, [1] * 6, nz=n)
+ang = np.zeros((6, 3), np.float32)
+for j, axis in enumerate((0, 1, 2, 1, 0, 2)):
+    ang[j, axis] = 10.0  # one sub-rotation
+b.iteration_setup(n, ang, positivity=False)
+F.fake_watch(b"k_shear", 16 * C.sizeof(Job))
+F.fake_clear_log()
+b.iterate(1, use_graph=False)
+strides = []
+for i in range(F.fake_launches()):
+    if b"k_shear" in F.fake_name(i):
+        jobs = (Job * 16).from_address(F.fake_arg(i))
+        strides.append([j.sc for j in jobs[:F.fake_blocks(i) // n]])
+b.close()
+report(strides=strides, bad=F.fake_bad())
+""")
+    assert r["bad"] == 0
+    jobs = [s for launch in r["strides"] for s in launch]
+    assert len(jobs) == 2 * 6 * 3  # there and back, six tilts, three shears that move anything
+    assert 1 not in jobs
