@@ -91,3 +91,22 @@ report(strides=strides, bad=F.fake_bad())
     jobs = [s for launch in r["strides"] for s in launch]
     assert len(jobs) == 2 * 6 * 3  # there and back, six tilts, three shears that move anything
     assert 1 not in jobs
+
+
+def test_sequential_pass_without_memory_for_its_slabs_runs_on_one_cta():
+    r = hostcuda.run("""
+got = {}
+for n in (24, 32, 48, 64, 96, 128, 160, 256):
+    s = sequential(n)
+    F.fake_clear_log()
+    F.fake_deny(n * n * 4 * 8)  # the slabs, [ns = 4][n][n] complex64
+    got[n] = [outcome(s.run, 1), outcome(s.step02, 0, n / 2.0, n / 2.0)]
+    F.fake_deny(8 * 3 * n * (8 if n in (24, 32, 64) else 16) // 32)  # one position's partial sums
+    got[n] += [outcome(s.step03), launched()]
+    F.fake_deny(0)
+    s.close()
+report(got=got)
+""")
+    for n, (run, forward, adjoint, names) in r["got"].items():
+        assert (run, forward, adjoint) == (0, 0, 0), n
+        assert sum("k_positions" in x for x in names) == 3 and not any("k_sequential" in x for x in names), n
