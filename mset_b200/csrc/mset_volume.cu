@@ -508,8 +508,10 @@ struct TvCluster {
             if (bytes > 220 * 1024 || !tv_cluster_pays(A, K, FISTA, march)) continue;
             auto k = k_tv_cluster<FISTA>;
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
-                (cl > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
-                return false;
+                (cl > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+                cudaGetLastError();  // the answer, not a later launch's error
+                continue;
+            }
             cfg.gridDim = dim3(cl);
             cfg.blockDim = dim3((unsigned)std::min(992L, (A + 31) / 32 * 32) + 32);
             cfg.dynamicSmemBytes = (size_t)bytes;
@@ -521,7 +523,9 @@ struct TvCluster {
             cfg.attrs = at;
             cfg.numAttrs = 1;
             int n = 0;
-            if (cl <= 8 || (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0)) return true;
+            if (cl <= 8) return true;
+            if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) cudaGetLastError();
+            else if (n > 0) return true;
         }
         return false;
     }

@@ -725,7 +725,9 @@ bool seq_fits() {
         auto k = k_sequential<G, kMSET, kREF, kSeq>;
         SeqConfig<G> c;
         int n = 0;
-        return c.prepare(k, nullptr) == 0 && cudaOccupancyMaxActiveClusters(&n, k, &c.cfg) == cudaSuccess && n > 0;
+        if (c.prepare(k, nullptr) == 0 && cudaOccupancyMaxActiveClusters(&n, k, &c.cfg) == cudaSuccess) return n > 0;
+        cudaGetLastError();  // the query's error is the answer, not a later launch's
+        return false;
     } else {
         return true;
     }

@@ -110,3 +110,17 @@ report(got=got)
     for n, (run, forward, adjoint, names) in r["got"].items():
         assert (run, forward, adjoint) == (0, 0, 0), n
         assert sum("k_positions" in x for x in names) == 3 and not any("k_sequential" in x for x in names), n
+
+
+def test_a_device_without_clusters_of_16_is_no_error():
+    """the query for them fails there: the smaller cluster, or one CTA, runs
+    and the query's error is not taken for a later launch's"""
+    r = hostcuda.run("""
+F.fake_clusters(-1)
+s = sequential(96)
+got = [s.sequential_split(), outcome(s.run, 1), outcome(s.tv, np.zeros((16, 16, 16), np.float32), 0.1, 2, True),
+       outcome(s.tv, np.zeros((48, 48, 48), np.float32), 0.1, 2, True)]
+report(got=got, names=launched())
+""")
+    assert r["got"] == [1, 0, 0, 0]
+    assert any("k_tv_cluster" in x for x in r["names"]) and not any("k_sequential" in x for x in r["names"])
