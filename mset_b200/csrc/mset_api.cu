@@ -77,6 +77,7 @@ struct DevBuf {
         if (e == cudaSuccess) n = count;
         return e;
     }
+    cudaError_t at_least(size_t count) { return n < count ? ensure(count) : cudaSuccess; }
 };
 
 }  // namespace
@@ -154,6 +155,7 @@ struct mset_session {
     cudaGraphExec_t graph_exec = nullptr;
     cudaGraph_t phase_graph[2] = {nullptr, nullptr};
     cudaGraphExec_t phase_exec[2] = {nullptr, nullptr};
+    std::vector<const void *> graph_sig;  // pointers and shapes the captured graphs were built on
     int grid_cache = 0;
     // TV work buffers
     DevBuf<float> tv_in, tv_out, tv_P, tv_Y, tv_Y2, tv_D;
@@ -1349,11 +1351,18 @@ int mset_rotate_volume(mset_session *s, const float *vol_in, float *vol_out, int
 }
 
 // ---- TV / TV-FISTA ----------------------------------------------------------
-// the second momentum field where it saves a kernel per iteration; without the
-// memory for it TV runs on what it has
-static int tv_second(mset_session *s, int n1, int n2, int n3, int fista) {
-    const size_t want = tv_wants_second(n1, n2, n3, fista != 0) ? 3 * (size_t)n1 * n2 * n3 : 0;
-    const cudaError_t e = s->tv_Y2.n < want ? s->tv_Y2.ensure(want) : cudaSuccess;
+// TV work buffers of V voxels.  exact: of that size, or of the iteration's where a
+// session that iterates needs more; else what is there is kept if it is enough.
+// The second momentum field comes where it saves a kernel per iteration; without
+// the memory for it TV runs on what it has.
+static int tv_prepare(mset_session *s, int n1, int n2, int n3, int fista, bool exact) {
+    size_t V = (size_t)n1 * n2 * n3;
+    const size_t second = tv_wants_second(n1, n2, n3, fista != 0) ? 3 * V : 0;
+    if (s->it_ready && s->it_tv) V = std::max(V, (size_t)s->nv1 * s->nv2 * s->nv3);
+    for (DevBuf<float> *b : {&s->tv_in, &s->tv_out, &s->tv_D}) CK(exact ? b->ensure(V) : b->at_least(V));
+    for (DevBuf<float> *b : {&s->tv_P, &s->tv_Y}) CK(exact ? b->ensure(3 * V) : b->at_least(3 * V));
+    CK(s->tv_err.ensure(1));
+    const cudaError_t e = s->tv_Y2.at_least(second);
     if (e == cudaErrorMemoryAllocation) cudaGetLastError();
     else if (e != cudaSuccess) return cuda_fail(e, "allocating the TV work field");
     return 0;
@@ -1368,13 +1377,7 @@ int mset_tv(mset_session *s, float *vol, int n1, int n2, int n3, double lambda, 
     int rc = set_device(s);
     if (rc) return rc;
     const size_t V = (size_t)n1 * n2 * n3;
-    CK(s->tv_in.ensure(V));
-    CK(s->tv_out.ensure(V));
-    CK(s->tv_P.ensure(3 * V));
-    CK(s->tv_Y.ensure(3 * V));
-    CK(s->tv_D.ensure(V));
-    CK(s->tv_err.ensure(1));
-    rc = tv_second(s, n1, n2, n3, fista);
+    rc = tv_prepare(s, n1, n2, n3, fista, true);
     if (rc) return rc;
     CK(cudaMemcpyAsync(s->tv_in.p, vol, sizeof(float) * V, cudaMemcpyHostToDevice, s->st));
     CK(cudaMemsetAsync(s->tv_err.p, 0, sizeof(double), s->st));
@@ -1401,6 +1404,36 @@ static void drop_graph(mset_session *s) {
         s->phase_exec[p] = nullptr;
         s->phase_graph[p] = nullptr;
     }
+    s->graph_sig.clear();
+}
+
+// Before an iteration is recorded or replayed: its work buffers and the twiddles
+// of its side are there (rotations and TV of other sizes on the same session
+// share them), and a graph captured on other buffers is dropped.
+static int iteration_prepare(mset_session *s) {
+    const size_t nvox = (size_t)s->nv1 * s->nv2 * s->nv3;
+    int rc = s->nv > 0 ? rot_prepare(s, s->nv) : rot_prepare3(s, s->nv1, s->nv2, s->nv3);
+    if (!rc && s->nv > 0 && s->rot_S.n < s->rot_group * nvox) rc = rot_prepare_group(s, s->nv, (int)s->tilts.size());
+    if (!rc && s->it_tv) rc = tv_prepare(s, s->nv1, s->nv2, s->nv3, s->it_tv_fista, false);
+    if (rc) return rc;
+    std::vector<const void *> sig;
+    for (const DevBuf<float> *b : {&s->rec, &s->gvol, &s->mx, &s->tv_in, &s->tv_out, &s->tv_P, &s->tv_Y, &s->tv_Y2, &s->tv_D})
+        sig.push_back(b->p);
+    for (const DevBuf<double> *b : {&s->gacc, &s->err_hist, &s->tv_hist, &s->tv_err, &s->err}) sig.push_back(b->p);
+    for (const DevBuf<float2> *b : {&s->rot_S, &s->rot_tw, &s->pscr, &s->psep, &s->twn, &s->save}) sig.push_back(b->p);
+    for (const DevBuf<unsigned> *b : {&s->it_counter, &s->mx_bits, &s->counter}) sig.push_back(b->p);
+    sig.push_back(s->d_tilts.p);
+    sig.push_back(s->items.p);
+    sig.push_back(s->plan.ops);
+    for (int v : {s->grid_cache, s->ckpt, s->rot_group, s->total_pos, s->hist_cap})
+        sig.push_back(reinterpret_cast<const void *>((intptr_t)v));
+    for (const TiltBufs &t : s->tilts)
+        for (const void *p : {(const void *)t.V.p, (const void *)t.Q.p, (const void *)t.sx.p, (const void *)t.sy.p,
+                              (const void *)t.grad.p, (const void *)t.qacc.p, (const void *)t.posdir.p})
+            sig.push_back(p);
+    if (sig != s->graph_sig) drop_graph(s);
+    s->graph_sig.swap(sig);
+    return 0;
 }
 
 namespace {
@@ -1434,6 +1467,7 @@ int mset_batch_iteration_setup_nd(mset_session *s, const mset_iter_args *a, int 
     rc = cubic ? rot_prepare(s, nv1) : rot_prepare3(s, nv1, nv2, nv3);
     if (!rc && cubic) rc = rot_prepare_group(s, nv1, J);
     if (rc) return rc;
+    s->it_ready = false;  // until the new buffers are all there
     const double v1[3] = {a->vec1[0], a->vec1[1], a->vec1[2]}, v2[3] = {a->vec2[0], a->vec2[1], a->vec2[2]},
                  v3[3] = {a->vec3[0], a->vec3[1], a->vec3[2]};
     s->plan_inv.resize(J);
@@ -1461,13 +1495,7 @@ int mset_batch_iteration_setup_nd(mset_session *s, const mset_iter_args *a, int 
     s->it_tv_fista = a->tv_fista ? 1 : 0;
     s->it_tv_lambda = a->tv_lambda;
     if (s->it_tv) {
-        CK(s->tv_in.ensure(V));
-        CK(s->tv_out.ensure(V));
-        CK(s->tv_P.ensure(3 * V));
-        CK(s->tv_Y.ensure(3 * V));
-        CK(s->tv_D.ensure(V));
-        CK(s->tv_err.ensure(1));
-        rc = tv_second(s, nv1, nv2, nv3, s->it_tv_fista);
+        rc = tv_prepare(s, nv1, nv2, nv3, s->it_tv_fista, true);
         if (rc) return rc;
     }
     CK(cudaStreamSynchronize(s->st));
@@ -1581,8 +1609,9 @@ int mset_batch_iterate(mset_session *s, int niter, int use_graph, double *err_ou
         CK(s->err_hist.ensure((size_t)cap * J));
         CK(s->tv_hist.ensure(cap));
         s->hist_cap = cap;
-        drop_graph(s);
     }
+    rc = iteration_prepare(s);
+    if (rc) return rc;
     CK(cudaMemsetAsync(s->it_counter.p, 0, sizeof(unsigned), s->st));
     CK(cudaStreamSynchronize(s->st));
     if (use_graph) {
@@ -1704,6 +1733,8 @@ int mset_batch_iterate_bls(mset_session *s, int niter, double bls_parameter, dou
     CK(s->bls_rec.ensure(V));
     CK(s->bls_q.ensure(std::max<size_t>(1, n2 * J)));
     CK(s->bls_pos.ensure(std::max<size_t>(1, 2 * (size_t)s->total_pos)));
+    rc = iteration_prepare(s);
+    if (rc) return rc;
     // the step sizes change below: graphs captured with the old ones are stale
     drop_graph(s);
     const float step0_orig = s->step[0];
@@ -1774,6 +1805,8 @@ int mset_batch_iterate_phase(mset_session *s, int phase, int use_graph) {
             s->hist_cap = 1;
         }
     }
+    rc = iteration_prepare(s);
+    if (rc) return rc;
     // the history slot of a single phase call is always the first
     CK(cudaMemsetAsync(s->it_counter.p, 0, sizeof(unsigned), s->st));
     if (use_graph) {

@@ -1,6 +1,8 @@
 """Host code of the library that no device can be made to reach: on a CUDA
 runtime of host memory (hostcuda.py)."""
-from mset_b200 import MSET_E_CUDA, MSET_E_STATE
+import pytest
+
+from mset_b200 import MSET_E_CUDA, MSET_E_NOMEM, MSET_E_STATE
 from tests import hostcuda
 
 
@@ -124,3 +126,85 @@ report(got=got, names=launched())
 """)
     assert r["got"] == [1, 0, 0, 0]
     assert any("k_tv_cluster" in x for x in r["names"]) and not any("k_sequential" in x for x in r["names"])
+
+
+# an iterating session of side `edge`, and other calls on it in between
+ITERATING = """
+def iterating(edge, window, tilts=3):
+    b = batched(window, [1] * tilts, nz=edge)
+    b.iteration_setup(edge, 10.0 * np.arange(3 * tilts, dtype=np.float32).reshape(tilts, 3) + 7, positivity=False,
+                      tv_lambda=0.1, tv_iter=2, tv_fista=True)
+    return b
+
+def tv(b, *shape):
+    b._lib.mset_tv(b._h, flat(*shape).ctypes.data_as(C.POINTER(C.c_float)), shape[2], shape[1], shape[0], 0.1, 2, 1, None)
+
+def rotate(b, n):
+    f = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))
+    v, e = flat(n, n, n), np.eye(3, dtype=np.float32)
+    return b._lib.mset_rotate_volume(b._h, f(v), f(v), n, f(e[0].copy()), f(e[1].copy()), f(e[2].copy()), 0.0, 20.0, 0.0, 0)
+
+class Job(C.Structure):  # ShearJob of csrc/mset_rotate.cu
+    _fields_ = [("S", C.c_void_p), ("cx", C.c_double), ("cy", C.c_double), ("sx", C.c_int), ("sy", C.c_int),
+                ("sc", C.c_int), ("real", C.c_int)]
+
+def stale(n):
+    "shears of side n that were handed a work volume outside live memory"
+    live = [(F.fake_alloc(i), F.fake_alloc_bytes(i)) for i in range(F.fake_allocs())]
+    bad = 0
+    for i in range(F.fake_launches()):
+        if b"k_shear" in F.fake_name(i):
+            for j in (Job * 16).from_address(F.fake_arg(i))[:F.fake_blocks(i) // n]:
+                bad += not any(p <= j.S and j.S + 8 * n ** 3 <= p + m for p, m in live)
+    return bad
+
+F.fake_watch(b"k_shear", 16 * C.sizeof(Job))
+"""
+
+
+@pytest.mark.parametrize("graph", [False, True], ids=["launches", "graph"])
+@pytest.mark.parametrize("between", ["tv(b, 24, 24, 24)", "tv(b, 64, 64, 64)", "rotate(b, 24)", "rotate(b, 96)",
+                                     "(tv(b, 50, 50, 60), rotate(b, 64), tv(b, 8, 8, 8))"])
+def test_iterations_keep_their_buffers_whatever_runs_between(between, graph):
+    r = hostcuda.run(ITERATING + f"""
+b = iterating(48, 48)
+b.iterate(1, use_graph={graph})
+{between}
+F.fake_clear_log()
+before = F.fake_bad()
+b.iterate(1, use_graph={graph})
+report(before=before, bad=F.fake_bad(), stale=stale(48), n=F.fake_launches())
+""")
+    assert r == dict(before=0, bad=0, stale=0, n=r["n"]) and r["n"] > 10
+
+
+def test_twiddles_of_the_iteration_s_side_are_back_after_another_rotation():
+    r = hostcuda.run(ITERATING + """
+b = iterating(48, 48)
+b.iterate(1, use_graph=False)
+tw = {n: np.exp(-2j * np.pi * np.outer(np.arange(n // 16), np.arange(16)) / n).astype(np.complex64) for n in (48,)}
+def tables():
+    "live allocations that start with the side's table [k2][n1]"
+    want, m = tw[48].ravel(), 0
+    for i in range(F.fake_allocs()):
+        if F.fake_alloc_bytes(i) == want.nbytes:
+            got = np.frombuffer((C.c_char * want.nbytes).from_address(F.fake_alloc(i)), np.complex64)
+            m += np.allclose(got, want, atol=1e-6)
+    return m
+first = tables()
+rotate(b, 64)
+b.iterate(1, use_graph=False)
+report(first=first, after=tables())
+""")
+    assert r["first"] > 0 and r["after"] == r["first"]
+
+
+def test_a_setup_that_failed_half_way_leaves_nothing_to_iterate():
+    r = hostcuda.run(ITERATING + """
+b = iterating(48, 48)
+F.fake_deny(8 * 48 * 24 * 24)  # the gradient sum of a smaller reconstruction, FP64
+again = outcome(b.iteration_setup, (48, 24, 24), np.zeros((3, 3), np.float32))
+F.fake_deny(0)
+report(again=again[0], then=outcome(b.iterate, 1)[0], bad=F.fake_bad())
+""")
+    assert r == dict(again=MSET_E_NOMEM, then=MSET_E_STATE, bad=0)
