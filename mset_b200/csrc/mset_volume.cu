@@ -573,15 +573,18 @@ int tv_prox(const TvArgs &a, cudaStream_t st) {
         if ((e = cudaMemsetAsync(a.Y, 0, sizeof(float) * 3 * V, st)) != cudaSuccess) return (int)e;
         const int q1 = std::max(1, a.n1 / 4), ty = std::max(1, std::min(128 / q1, a.n2));
         const int tiles = (a.n2 + ty - 1) / ty;
+        // chunks of zc slices: every wave of resident CTAs (80 registers: 25 warps an
+        // SM) takes a chunk's chain, 1.4 us a slice and 0.9 slices' time to start,
+        // however full it is; what moves through memory comes on top of that
+        // alike for every zc.  Within 3% of the best zc at each of 34 volumes timed,
+        // 4x4x1000 to 256^3 (128^3: 16.4 us an iteration at zc = 5, one wave; 17.1 at
+        // 3, two; 19.0 at 7; 19.5 at 1, five; 160x160x96: 21.0 at 6, 24.4 at 8;
+        // 192x192x96: 32.7 at 8, 43.6 at 16; 256x256x64: 38.4 at 5, 42.2 at 13)
+        const double wave = 148.0 * (25 / ((q1 * ty + 31) / 32));
         int zc = 1;
         double best = 0;
         for (int c = 1; c <= std::min(16, a.n3); ++c) {
-            // chunks of c slices (0.6 more for a chunk's start) in waves of the
-            // 6 CTAs an SM holds; a wave less than two thirds full takes as
-            // long as one, half of a last wave's empty places are lost (128^3:
-            // 17.6 us at c = 5, 0.94 waves; 21.2 at 4, 1.15; 18.0 at 3; 24.0 at 1)
-            const double w = (double)tiles * ((a.n3 + c - 1) / c) / (148.0 * 6.0), up = std::ceil(w);
-            const double cost = (c + 0.6) * (w <= 1.0 ? std::max(w, 0.65) : 0.5 * (w + up));
+            const double cost = (c + 0.9) * std::ceil(tiles * ((a.n3 + c - 1) / c) / wave);
             if (c == 1 || cost < best) {
                 best = cost;
                 zc = c;

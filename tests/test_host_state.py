@@ -208,3 +208,16 @@ F.fake_deny(0)
 report(again=again[0], then=outcome(b.iterate, 1)[0], bad=F.fake_bad())
 """)
     assert r == dict(again=MSET_E_NOMEM, then=MSET_E_STATE, bad=0)
+
+
+@pytest.mark.parametrize("shape,zc", [((128, 128, 128), 5), ((96, 160, 160), 6), ((64, 256, 256), 5),
+                                      ((96, 192, 192), 8), ((192, 256, 256), 15), ((1000, 8, 8), 1)])
+def test_march_chunks_that_measured_fastest(shape, zc):
+    r = hostcuda.run(f"""
+with Session() as s:
+    s.tv(np.zeros({shape}, np.float32), 0.1, 1, True)
+report(blocks=[F.fake_blocks(i) for i in range(F.fake_launches()) if b"k_tv_march" in F.fake_name(i)])
+""")
+    n3, n2, n1 = shape
+    rows = min(128 // (n1 // 4), n2)  # of a CTA
+    assert r["blocks"] == [-(-n2 // rows) * -(-n3 // zc)]
