@@ -432,8 +432,8 @@ int seq_prepare(mset_session *s, int method, int npos, bool *cluster) {
         TiltBufs &t = s->tilts[0];
         const size_t parts = (size_t)(2 * std::max(1, npos) + 1) * s->seq->warps;
         const size_t slabs = method == kSSET ? 1 : s->ns;
-        cudaError_t e = t.T.n < n2 * slabs ? t.T.ensure(n2 * s->ns) : cudaSuccess;
-        if (e == cudaSuccess && s->seq_part.n < parts) e = s->seq_part.ensure(parts);
+        cudaError_t e = t.T.at_least(n2 * slabs);
+        if (e == cudaSuccess) e = s->seq_part.at_least(parts);
         if (e == cudaErrorMemoryAllocation && s->plan.ops->seq) {
             cudaGetLastError();
             *cluster = false;

@@ -221,3 +221,13 @@ report(blocks=[F.fake_blocks(i) for i in range(F.fake_launches()) if b"k_tv_marc
     n3, n2, n1 = shape
     rows = min(128 // (n1 // 4), n2)  # of a CTA
     assert r["blocks"] == [-(-n2 // rows) * -(-n3 // zc)]
+
+
+def test_single_slice_sequential_pass_asks_for_one_slab():
+    r = hostcuda.run("""
+s = sequential(64)
+F.fake_deny(64 * 64 * 4 * 8)  # [nz = 4][n][n] complex64
+F.fake_clear_log()
+report(run=outcome(s.run, 2), names=launched())
+""")
+    assert r["run"] == 0 and any("k_sequential" in x for x in r["names"])
