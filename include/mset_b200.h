@@ -410,9 +410,9 @@ int mset_rotate_volume_nd(mset_session *s, const float *vol_in, float *vol_out, 
  * output = input - lambda div(P), tv_error = lambda * sum |grad(output)|.
  * vol: host [n3][n2][n1] float, replaced by the output.  Dual variables in
  * FP32 (the reference's arithmetic is single once it meets the single input),
- * FISTA momentum step in FP64, error in FP64.  Scratch: 9 (TV) to 13 (FISTA)
- * floats per voxel; without memory for the last three FISTA runs on two kernels
- * per iteration instead of one. */
+ * FISTA momentum step in FP64, error in FP64.  Scratch: 9 floats per voxel, 12
+ * for FISTA on volumes that take one kernel per iteration; without memory for
+ * the last three it takes two. */
 int mset_tv(mset_session *s, float *vol, int n1, int n2, int n3, double lambda, int niter, int fista,
             double *tv_error);
 

@@ -430,10 +430,9 @@ int seq_prepare(mset_session *s, int method, int npos, bool *cluster) {
     *cluster = seq_on_cluster(s);
     if (*cluster) {
         TiltBufs &t = s->tilts[0];
-        const size_t parts = (size_t)(2 * std::max(1, npos) + 1) * s->seq->warps;
         const size_t slabs = method == kSSET ? 1 : s->ns;
         cudaError_t e = t.T.at_least(n2 * slabs);
-        if (e == cudaSuccess) e = s->seq_part.at_least(parts);
+        if (e == cudaSuccess) e = s->seq_part.at_least(seq_partials(std::max(1, npos), s->seq->warps));
         if (e == cudaErrorMemoryAllocation && s->plan.ops->seq) {
             cudaGetLastError();
             *cluster = false;

@@ -15,13 +15,18 @@ namespace mset {
 //  24, 32  one shape (192 threads at 24: 81 us at P = 148, 648 at 3000, 24
 //          slabs; 64 threads took 138 and 805)
 //  48      192 threads with 128 registers x 2 CTAs up to 2 positions per SM
-//          (244 against 271 at P = 296), x 4 above (1286 against 1517 at 2000)
-//  64      256 threads x 2 CTAs up to 6 positions per SM (349 against 411 at P =
-//          296, 804 against 846 at 740), 128 x 4 above (9645 against 10574 at P
-//          = 8000, 32 slabs)
-//  96      384 threads x 2 CTAs (80 registers; 3600 at P = 1184, 32 slabs,
-//          against 4380 with one CTA and 128 registers); one CTA up to one
-//          position per SM (584 against 635 at P = 148)
+//          (314 against 363 at P = 296, 32 slabs; ahead at each of five counts
+//          from 0.25 an SM on), x 4 above (448 against 498 at 2.5 an SM, 1691
+//          against 1950 at 13.5; ahead at each of eight counts)
+//  64      256 threads x 2 CTAs up to 6 positions per SM, 128 x 4 above.  By how
+//          their last waves fill they lead in turn between 2 and 6 (32 slabs:
+//          450 against 521 at 2, 670 / 646 at 3, 854 / 806 at 4, 1021 / 1089 at 5,
+//          1245 / 1194 at 6); below the first is ahead (308 / 449 at 1), above the
+//          second (1372 / 1334 at 6.5, 1761 / 1576 at 8, 10248 / 9385 at 54)
+//  96      384 threads x 2 CTAs (80 registers; 984 against 1105 with one CTA and
+//          128 registers at 1.25 positions per SM, 32 slabs, 3613 against 4396 at
+//          8; ahead at each of nine counts); one CTA up to one position per SM
+//          (586 against 643 at 1, 552 against 599 at 0.25)
 //  128     the three-phase shape; the two-pass one serves the sequential
 //          sessions
 //  256     the saved-wave rows staged by bulk copies (1.443 s against 1.474 s

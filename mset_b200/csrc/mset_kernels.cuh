@@ -105,6 +105,11 @@ struct SeqOps {
     int (*positions)(int method, int adjoint, int mode, const LaunchArgs &a, cudaStream_t st);
 };
 
+// doubles the sequential cluster kernels leave their partial sums in
+// (LaunchArgs::seq_part): per position and warp of the cluster the two
+// scan-position sums, then per warp the error sum
+inline size_t seq_partials(int npos, int warps) { return (size_t)(2 * npos + 1) * warps; }
+
 // host-side launchers (return cudaError_t as int)
 struct Plan {
     int n, r1, ry1, nt;

@@ -36,9 +36,10 @@
 // stays in registers for the whole call, the probe spectrum in shared memory;
 // positions' sums are written per warp and added up once at the end.
 //
-// What bounds it: the chain.  Of about 6000 cycles per slab and direction at
-// 128^2 (8 CTAs of 16 rows) the two exchanges take 3600 (16 KB each way per
-// CTA), the passes 2200; at 64^2 (8 CTAs of 8 rows) 1500 and 1400 of 3050.
+// What bounds it: the chain.  Of 6030 cycles per slab and direction at 128^2 (8
+// CTAs of 16 rows, 16 KB each way per CTA) the pushes and waits take 2860, the
+// slots between them 1060, the passes 2050; of 3050 at 64^2 (8 CTAs of 8 rows)
+// 1080, 720 and 1190.
 // The times per window and cluster size stand at MSET_SEQ_FIELDS in
 // mset_dispatch.cu.
 #pragma once
@@ -98,10 +99,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity)
     }
     return false;
 }
-
-// doubles the sequential kernels leave their partial sums in: per position and
-// warp the two scan-position sums, then per warp the error sum
-__host__ __device__ inline size_t seq_partials(int npos, int warps) { return (size_t)(2 * npos + 1) * warps; }
 
 template <class G, int METHOD, int ADJ, int MODE>
 struct SeqKernel {
