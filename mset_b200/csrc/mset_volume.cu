@@ -154,12 +154,12 @@ __device__ __forceinline__ void tv_project(float q1, float q2, float q3, float &
 // chain of a step), 16.3 -> 10.0 at 96^3, 12.3 -> 6.1 at 64^3.
 //
 // Each iteration's kernel is set up while the one before drains (programmatic
-// dependent launch; the wait stands before the first access): 108.2, 18.6, 8.8
-// and 3.9 us there, 3.4 against 6.1 at 48^3; inside a captured iteration, whose
-// launches cost less, 2.5% of it at 48^3 and 0.5 to 2% above.  The kernels do not
-// signal early: CTAs of the next iteration then take places among the running
-// ones, whose neighbours share slices in L2 (129.7 us at 256 x 256 x 192, 19.8 at
-// 128^3).
+// dependent launch; the wait stands before the first access): 108.2, 18.6 (16.4
+// since the chunks go by whole waves, tv_prox), 8.8 and 3.9 us there, 3.4 against
+// 6.1 at 48^3; inside a captured iteration, whose launches cost less, 2.5% of it at
+// 48^3 and 0.5 to 2% above.  The kernels do not signal early: CTAs of the next
+// iteration then take places among the running ones, whose neighbours share slices
+// in L2 (129.7 us at 256 x 256 x 192, 19.8 at 128^3).
 struct Quad {
     float v[4];
 };
